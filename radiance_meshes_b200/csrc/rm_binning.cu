@@ -1176,9 +1176,9 @@ int rm_launch_build_lists(const int32_t* rect, const int32_t* tile_ranges, int64
   {
     RmProfScope prof("k_region_pairs", st);
     auto kernel = P.items == 4 ? rm::k_region_pairs<4> : rm::k_region_pairs<16>;
-    rm_count_launch(), kernel<<<P.nblk, rm::kBinThreads, 0, st>>>(
-        cum, order, (int)T, &counters->n_visible, ranked, P.reg_w, n_region_keys, P.passes, P.bits, digit_total, pairs[0],
-        reinterpret_cast<uint4*>(sb + P.zero), (int64_t)(P.zero_bytes / sizeof(uint4)));
+    RM_CUDA_CHECK(rm_launch(kernel, P.nblk, rm::kBinThreads, 0, st, cum, order, (int)T, &counters->n_visible, ranked,
+                            P.reg_w, n_region_keys, P.passes, P.bits, digit_total, pairs[0],
+                            reinterpret_cast<uint4*>(sb + P.zero), (int64_t)(P.zero_bytes / sizeof(uint4))));
   }
   {
     RmProfScope prof("k_region_pass", st);

@@ -28,14 +28,11 @@ static inline bool rm_aligned16(const void* p) { return (reinterpret_cast<uintpt
 // many of this library's kernels ran inside a timed region.
 void rm_count_launch();
 
-// Launch of a kernel that begins with rm::after_previous(), behind a kernel that the same call of the library has launched on
-// the same stream: its blocks are placed while the last blocks of that kernel still run, and wait there for its end.  Never for
-// the first launch of a call, which may have to wait for copies and events of the caller's.  Only for `items` (tets or pairs)
-// up to kFewItems, where the 2 to 3 us between the kernels count (60k tets, 203 x 317 pixels: frame 209 -> 194 us); the
-// waiting blocks of larger grids hold back more than that (600k tets, 800 x 800: 687 -> 699 us).
-constexpr int64_t kFewItems = 1 << 17;
+// All launches go through these two, which return the launch's own error: what follows on a kernel that did not start would
+// run on memory that nobody has written.
 template <typename... P, typename... A>
-cudaError_t rm_launch_behind(int64_t items, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+cudaError_t rm_launch_config(bool behind, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+                             A... args) {
   rm_count_launch();
   cudaLaunchAttribute attribute = {};
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -46,8 +43,24 @@ cudaError_t rm_launch_behind(int64_t items, void (*kernel)(P...), unsigned block
   config.dynamicSmemBytes = smem;
   config.stream = st;
   config.attrs = &attribute;
-  config.numAttrs = items <= kFewItems ? 1 : 0;
+  config.numAttrs = behind ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t rm_launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+  return rm_launch_config(false, kernel, blocks, threads, smem, st, args...);
+}
+
+// Launch of a kernel that begins with rm::after_previous(), behind a kernel that the same call of the library has launched on
+// the same stream: its blocks are placed while the last blocks of that kernel still run, and wait there for its end.  Never for
+// the first launch of a call, which may have to wait for copies and events of the caller's.  Only for `items` (tets or pairs)
+// up to kFewItems, where the 2 to 3 us between the kernels count (60k tets, 203 x 317 pixels: frame 209 -> 194 us); the
+// waiting blocks of larger grids hold back more than that (600k tets, 800 x 800: 687 -> 699 us).
+constexpr int64_t kFewItems = 1 << 17;
+template <typename... P, typename... A>
+cudaError_t rm_launch_behind(int64_t items, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+                             A... args) {
+  return rm_launch_config(items <= kFewItems, kernel, blocks, threads, smem, st, args...);
 }
 
 // Optional per-kernel timing (rm_profile_enable): a scope records a CUDA event

@@ -63,7 +63,6 @@ int rm_launch_multimem_sum(float* mc, int64_t float_begin, int64_t float_end, in
   const int64_t want = (e - b + rm::kSumThreads * rm::kSumUnroll - 1) / (rm::kSumThreads * rm::kSumUnroll);
   const unsigned blocks = (unsigned)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
   RmProfScope prof("k_multimem_sum", st);
-  rm_count_launch(), rm::k_multimem_sum<<<blocks, rm::kSumThreads, 0, st>>>(mc, b, e);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_multimem_sum, blocks, rm::kSumThreads, 0, st, mc, b, e));
   return RM_OK;
 }

@@ -762,7 +762,7 @@ int rm_launch_project(const int32_t* indices, int64_t T, const float* vertices, 
   {
     RmProfScope prof("k_project", st);
     auto kernel = fisheye ? rm::k_project<true> : rm::k_project<false>;
-    rm_count_launch(), kernel<<<(unsigned)blocks, rm::kProjectThreads, 0, st>>>(indices, T, vertices, V, *cam, o);
+    RM_CUDA_CHECK(rm_launch(kernel, (unsigned)blocks, rm::kProjectThreads, 0, st, indices, T, vertices, V, *cam, o));
   }
   {
     RmProfScope prof("k_project_deferred", st);
@@ -779,7 +779,7 @@ int rm_launch_vertex_backward(const int32_t* indices, const float* vertices, int
   if (T == 0) return RM_OK;
   unsigned blocks = (unsigned)((T + 255) / 256);
   RmProfScope prof("k_vertex_backward", st);
-  rm_count_launch(), rm::k_vertex_backward<<<blocks, 256, 0, st>>>(indices, vertices, T, *cam, tiles_touched, g_vs, g_cc, vgrad);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_vertex_backward, blocks, 256, 0, st, indices, vertices, T, *cam, tiles_touched, g_vs, g_cc,
+                          vgrad));
   return RM_OK;
 }

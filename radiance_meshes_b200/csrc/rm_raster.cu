@@ -1723,16 +1723,15 @@ int rm_launch_distortion_loss(const float* dist, int64_t n, float* partials, flo
   const int64_t want = (n + 4 * rm::kLossThreads - 1) / (4 * rm::kLossThreads);  // four pixels per thread, or more
   const int blocks = (int)(want < RM_LOSS_PARTIALS ? want : RM_LOSS_PARTIALS);
   RmProfScope prof("k_distortion_loss(2 launches)", st);
-  rm_count_launch(), rm::k_distortion_loss<<<blocks, rm::kLossThreads, 0, st>>>(dist, n, partials);
+  RM_CUDA_CHECK(rm_launch(rm::k_distortion_loss, blocks, rm::kLossThreads, 0, st, dist, n, partials));
   RM_CUDA_CHECK(rm_launch_behind(blocks, rm::k_distortion_loss_mean, 1, rm::kLossThreads, 0, st, partials, blocks, n, loss));
   return RM_OK;
 }
 
 int rm_launch_distortion_loss_backward(const float* dist, int64_t n, const float* g_loss, float* g_dist, cudaStream_t st) {
   RmProfScope prof("k_distortion_loss_backward", st);
-  rm_count_launch(), rm::k_distortion_loss_backward<<<(unsigned)((n + rm::kLossThreads - 1) / rm::kLossThreads), rm::kLossThreads, 0,
-                                                     st>>>(dist, n, g_loss, g_dist);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_distortion_loss_backward, (unsigned)((n + rm::kLossThreads - 1) / rm::kLossThreads),
+                          rm::kLossThreads, 0, st, dist, n, g_loss, g_dist));
   return RM_OK;
 }
 
@@ -1753,9 +1752,9 @@ int rm_launch_pack(const int32_t* indices, const float* vertices, const float* c
                    cudaStream_t st) {
   if (T == 0) return RM_OK;
   RmProfScope prof("k_pack_records", st);
-  rm_count_launch(), rm::k_pack_records<<<(unsigned)((T + rm::kPackThreads - 1) / rm::kPackThreads), rm::kPackThreads, 0, st>>>(
-      indices, vertices, cell, T, V, *cam, tiles_touched, reinterpret_cast<float4*>(records), clear_a, clear_b);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_pack_records, (unsigned)((T + rm::kPackThreads - 1) / rm::kPackThreads), rm::kPackThreads,
+                          0, st, indices, vertices, cell, T, V, *cam, tiles_touched, reinterpret_cast<float4*>(records),
+                          clear_a, clear_b));
   return RM_OK;
 }
 
@@ -1792,17 +1791,16 @@ int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* r
   RmProfScope prof("k_forward", st);
   if (n_units > 8 * kWave && n_list >= 0) {
     const int long_blocks = 148 * 5, long_list = (int)std::min<int64_t>(3 * n_list / tiles, INT_MAX);
-    rm_count_launch(), rm::k_forward_long_first<<<blocks + long_blocks, threads, smem, st>>>(
-        list, tiles_list, recs, *cam, jit, img, dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units,
-        long_list, long_blocks);
+    RM_CUDA_CHECK(rm_launch(rm::k_forward_long_first, blocks + long_blocks, threads, smem, st, list, tiles_list, recs, *cam,
+                            jit, img, dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, long_list,
+                            long_blocks));
   } else {
     const bool pair = deal_by_pairs(n_units, tiles, n_list);
     auto kernel = pair ? rm::k_forward<rm::kColor, true> : rm::k_forward<rm::kColor, false>;
-    rm_count_launch(), kernel<<<pair ? pair_blocks : blocks, threads, smem, st>>>(
-        list, tiles_list, recs, *cam, jit, img, dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, 0.0f,
-        0.0f, rm::StatsArgs{});
+    RM_CUDA_CHECK(rm_launch(kernel, pair ? pair_blocks : blocks, threads, smem, st, list, tiles_list, recs, *cam, jit, img,
+                            dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, 0.0f, 0.0f,
+                            rm::StatsArgs{}));
   }
-  RM_CUDA_CHECK(cudaPeekAtLastError());
   return RM_OK;
 }
 
@@ -1818,12 +1816,10 @@ int rm_launch_forward_constant_color(const int32_t* list, const int32_t* ranges,
   const bool pair = deal_by_pairs(n_units, n_units / subs, n_list);
   if (pair) blocks = (unsigned)((n_units + rm::kWarpsPerBlock - 1) / rm::kWarpsPerBlock);
   auto kernel = pair ? rm::k_forward<rm::kConstColor, true> : rm::k_forward<rm::kConstColor, false>;
-  rm_count_launch(), kernel
-      <<<blocks, rm::kWarpsPerBlock * 32, rm::kWarpsPerBlock * sizeof(rm::FwdShared), st>>>(
-          list, reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
-          reinterpret_cast<float4*>(out_img), dist_img, n_contrib, nullptr, nullptr, nullptr, nullptr, subs, n_units,
-          pre_multi, ladder_p, rm::StatsArgs{});
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(kernel, blocks, rm::kWarpsPerBlock * 32, rm::kWarpsPerBlock * sizeof(rm::FwdShared), st, list,
+                          reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
+                          reinterpret_cast<float4*>(out_img), dist_img, n_contrib, nullptr, nullptr, nullptr, nullptr, subs,
+                          n_units, pre_multi, ladder_p, rm::StatsArgs{}));
   return RM_OK;
 }
 
@@ -1843,13 +1839,12 @@ int rm_launch_backward_constant_color(const int32_t* list, const int32_t* ranges
   unit_grid(cam, &subs, &n_units, &blocks);
   if (n_units > 0) {
     RmProfScope prof("k_backward<constant colour>", st);
-    rm_count_launch(), rm::k_backward_cc<<<blocks, rm::kWarpsPerBlock * 32, 0, st>>>(
-        list, reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam,
-        reinterpret_cast<const float4*>(out_img), reinterpret_cast<const float4*>(dist_img), n_contrib,
-        reinterpret_cast<const float4*>(g_img), reinterpret_cast<const float4*>(g_dist), pre_multi, ladder_p, grec, subs,
-        n_units);
+    RM_CUDA_CHECK(rm_launch(rm::k_backward_cc, blocks, rm::kWarpsPerBlock * 32, 0, st, list,
+                            reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam,
+                            reinterpret_cast<const float4*>(out_img), reinterpret_cast<const float4*>(dist_img), n_contrib,
+                            reinterpret_cast<const float4*>(g_img), reinterpret_cast<const float4*>(g_dist),
+                            pre_multi, ladder_p, grec, subs, n_units));
   }
-  RM_CUDA_CHECK(cudaPeekAtLastError());
   return RM_OK;
 }
 
@@ -1868,11 +1863,10 @@ int rm_launch_tet_err(const int32_t* list, const int32_t* ranges, const float* r
   RM_CUDA_CHECK(cudaFuncSetAttribute(rm::k_forward<rm::kStats, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   RmProfScope prof("k_tet_err", st);
-  rm_count_launch(), rm::k_forward<rm::kStats, false><<<blocks, rm::kWarpsPerBlock * 32, smem, st>>>(
-      list, reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr, nullptr,
-      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, subs, n_units, 0.0f, 0.0f,
-      rm::StatsArgs{pixel_err, ssim_err, tet_err, tet_count});
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_forward<rm::kStats, false>, blocks, rm::kWarpsPerBlock * 32, smem, st, list,
+                          reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
+                          nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, subs, n_units, 0.0f, 0.0f,
+                          rm::StatsArgs{pixel_err, ssim_err, tet_err, tet_count}));
   return RM_OK;
 }
 
@@ -1904,9 +1898,8 @@ static int launch_clear(const RmHitList* hits, int64_t T, int64_t V, float* grec
   const int64_t n = (T > 3 * V ? T : 3 * V), per_block = 4 * rm::kClearThreads;
   if (n == 0) return RM_OK;
   RmProfScope prof("k_clear_flagged_rows", st);
-  rm_count_launch(), rm::k_clear_flagged_rows<<<(unsigned)((n + per_block - 1) / per_block), rm::kClearThreads, 0, st>>>(
-      hits->tet_flags, T, reinterpret_cast<float4*>(grec), vgrad, 3 * V);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_clear_flagged_rows, (unsigned)((n + per_block - 1) / per_block), rm::kClearThreads, 0, st,
+                          hits->tet_flags, T, reinterpret_cast<float4*>(grec), vgrad, 3 * V));
   return RM_OK;
 }
 
@@ -1927,11 +1920,10 @@ int rm_launch_backward_finish(const int32_t* indices, const float* vertices, con
                               float* vgrad, float* cgrad, cudaStream_t st) {
   if (t_end <= t_begin) return RM_OK;
   RmProfScope prof("k_backward_finish", st);
-  rm_count_launch(), rm::k_backward_finish<<<(unsigned)((t_end - t_begin + rm::kFinishThreads - 1) / rm::kFinishThreads),
-                                            rm::kFinishThreads, 0, st>>>(
-      indices, vertices, cell, t_begin, t_end, *cam, reinterpret_cast<const float4*>(grec), hits->tet_flags, vgrad,
-      cgrad);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_backward_finish,
+                          (unsigned)((t_end - t_begin + rm::kFinishThreads - 1) / rm::kFinishThreads), rm::kFinishThreads, 0, st,
+                          indices, vertices, cell, t_begin, t_end, *cam, reinterpret_cast<const float4*>(grec),
+                          hits->tet_flags, vgrad, cgrad));
   return RM_OK;
 }
 
@@ -1999,10 +1991,9 @@ extern "C" int rm_backward_static_scratch(const int32_t* sorted_tetra_idx, const
                             grad_distortion_img, scratch, n_tets, st);
   if (rc) return rc;
   RmProfScope prof2("k_backward_finish", st);
-  rm_count_launch(), rm::k_backward_finish<<<(unsigned)((n_tets + rm::kFinishThreads - 1) / rm::kFinishThreads), rm::kFinishThreads, 0, st>>>(
-      indices, vertices, cell_values, 0, n_tets, *cam, reinterpret_cast<const float4*>(scratch), hits->tet_flags,
-      vertices_grad, cell_values_grad);
-  RM_CUDA_CHECK(cudaPeekAtLastError());
+  RM_CUDA_CHECK(rm_launch(rm::k_backward_finish, (unsigned)((n_tets + rm::kFinishThreads - 1) / rm::kFinishThreads),
+                          rm::kFinishThreads, 0, st, indices, vertices, cell_values, 0, n_tets, *cam,
+                          reinterpret_cast<const float4*>(scratch), hits->tet_flags, vertices_grad, cell_values_grad));
   return RM_OK;
 }
 
