@@ -35,8 +35,6 @@ extern "C" {
 #define RM_STATUS_BAD_INDEX 4u    /* a tet names a vertex outside [0, n_vertices): the tet is treated as culled
                                      (the reference would read out of bounds) */
 
-#define RM_STATUS_INTERNAL 8u     /* a block of the rank sort waited in vain for another: the lists are not valid */
-
 /* Floats per packed tet record (24 used by the integration + 12 for the hull edge
  * lines of the projected tet, used to cull whole tiles) and per record-gradient row. */
 #define RM_RECORD_FLOATS 36
@@ -380,16 +378,20 @@ int64_t rm_launch_count(void);
  * - list cursors, hit-list slots, ids read from lists and the rows they address - is compared with the
  * extent of its array before the access; a violation sets a bit of a status word and the access is
  * skipped, nothing traps.
- *   rm_debug_bounds_checked: 1 in the checked build, 0 otherwise (the other two are no-ops then).
+ *   rm_debug_bounds_checked: 1 in the checked build, 0 otherwise (the others are no-ops then).
  *   rm_debug_set_extent(which, n): extent of a caller-owned array of the integration stages, whose
  *     entry points carry no lengths: 0 list entries, 1 tets, 2 vertices, 3 hit-list id slots,
  *     4 hit-list mask slots, 5 hit-list units.
  *   rm_debug_bounds_status: waits for the device, returns the status word and clears it (bit = access
  *     site; 0 = every checked access was inside its array).
+ *   rm_debug_recounted: waits for the device, returns and clears one bit for each kind of look-back word (1 rank
+ *     sort, 2 scan in rank order, 4 region sort, 8 tile lists) that a block has counted itself, which this build
+ *     does whenever a word is not there at first sight (the ordinary one after some 10 ms of waiting).
  */
 int rm_debug_bounds_checked(void);
 void rm_debug_set_extent(int which, int64_t n);
 uint32_t rm_debug_bounds_status(void);
+uint32_t rm_debug_recounted(void);
 
 #ifdef __cplusplus
 }

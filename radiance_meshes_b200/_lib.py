@@ -14,7 +14,6 @@ RM_GRAD_RECORD_FLOATS = 24
 RM_STATUS_NAN_VERTEX = 1
 RM_STATUS_KEY_OVERFLOW = 2
 RM_STATUS_BAD_INDEX = 4
-RM_STATUS_INTERNAL = 8
 
 # every symbol include/rm_b200.h declares
 SYMBOLS = ["rm_strerror", "rm_version", "rm_bin_workspace_bytes", "rm_list_scratch_bytes", "rm_project_and_bin", "rm_build_tile_lists",
@@ -22,7 +21,7 @@ SYMBOLS = ["rm_strerror", "rm_version", "rm_bin_workspace_bytes", "rm_list_scrat
            "rm_profile_read", "rm_backward_static_scratch", "rm_tet_err",
            "rm_activate_output", "rm_forward_constant_color", "rm_launch_count",
            "rm_backward_integrate", "rm_backward_finish", "rm_debug_bounds_checked", "rm_debug_set_extent",
-           "rm_debug_bounds_status", "rm_backward_constant_color", "rm_multimem_sum", "rm_project_and_bin_visible",
+           "rm_debug_bounds_status", "rm_debug_recounted", "rm_backward_constant_color", "rm_multimem_sum", "rm_project_and_bin_visible",
            "rm_pack_records_and_clear", "rm_forward_sized", "rm_forward_constant_color_sized", "rm_distortion_loss", "rm_distortion_loss_backward"]
 RM_STATIC_SCRATCH_MAX_TETS = 131072
 RM_ERR_STATIC_SCRATCH = -5
@@ -97,6 +96,7 @@ def load():
     lib.rm_debug_set_extent.restype = None
     lib.rm_debug_set_extent.argtypes = [C.c_int, i64]
     lib.rm_debug_bounds_status.restype = C.c_uint32
+    lib.rm_debug_recounted.restype = C.c_uint32
     for name in SYMBOLS:
         getattr(lib, name)
     _lib = lib

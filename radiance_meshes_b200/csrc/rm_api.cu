@@ -147,6 +147,7 @@ int rm_debug_bounds_checked(void) {
 }
 void rm_debug_set_extent(int which, int64_t n) { rm_debug_extent_raster(which, (long long)n); }
 uint32_t rm_debug_bounds_status(void) { return rm_bounds_status_raster() | rm_bounds_status_binning(); }
+uint32_t rm_debug_recounted(void) { return rm_take_recounted(); }
 
 void rm_profile_enable(int on) {
   std::lock_guard<std::mutex> lk(g_prof_mu);

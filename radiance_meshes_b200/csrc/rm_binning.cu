@@ -226,8 +226,23 @@ static_assert(kSortThreads == kJobThreads && kSortThreads == kScanThreads, "the 
 constexpr int sort_items(int64_t n) { return n <= 64 * 4 * kSortThreads ? 4 : 16; }
 constexpr uint32_t kCulledKey = 0xFFFFFFFFu;
 // Look-back words: 0 not there yet; n + 1 a block's own run of n; kRunEnd | n all runs up to and with the block's.
+// No wait decides a result: from a word on that is not there after kMaxPolls polls, a block counts what is missing
+// itself, from the other blocks' items, which nothing writes while the kernel runs (finish_look_back).
 constexpr uint32_t kRunEnd = 1u << 31;
-constexpr int kMaxPolls = 1 << 20;  // about a second per word; then the call reports RM_STATUS_INTERNAL
+#ifdef RM_BOUNDS_CHECK
+constexpr int kMaxPolls = 0;  // the checked build counts every word that is not there at first sight
+static __device__ unsigned g_recounted;
+#else
+constexpr int kMaxPolls = 1 << 14;  // about 10 ms per word
+#endif
+enum Recounted { kRecountRankPass = 1, kRecountRankRects = 2, kRecountRegionPass = 4, kRecountFineLists = 8 };
+__device__ __forceinline__ void note_recount(Recounted which) {
+#ifdef RM_BOUNDS_CHECK
+  atomicOr(&g_recounted, (unsigned)which);
+#else
+  (void)which;
+#endif
+}
 
 __global__ void __launch_bounds__(kSortThreads)
 k_digit_hist(const uint32_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist /* [4][kRadix], zeroed */, TileJob job) {
@@ -269,12 +284,28 @@ __device__ __forceinline__ void store_relaxed(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v));
 }
 
+// Sum of what the `blocks` blocks before `word` hold, on top of `before`, without waiting; count(b): what block b holds.
+template <typename F>
+__device__ __forceinline__ uint32_t finish_look_back(uint32_t before, const uint32_t* word, uint32_t blocks, int stride, F count) {
+#pragma unroll 1
+  while (blocks) {
+    --blocks;
+    word -= stride;
+    uint32_t v = load_relaxed(word);
+    if (v == 0u) v = count(blocks) + 1u;
+    if (v & kRunEnd) return before + (v ^ kRunEnd);
+    before += v - 1u;
+  }
+  return before;
+}
+
 // Sum of what the `blocks` blocks before `word` hold, the nearest first, `stride` words apart.  AHEAD words are asked for
 // at a time: blocks that run together all walk over each other's runs, one round trip to L2 per word otherwise.  Two are
 // best for the rank sort (30M tets: 1016, 934, 1041 us with 1, 2, 8), whose blocks hold many words each, eight for the
-// list build (passes 592 -> 520 us each, lists 1683 -> 1551 us).
-template <uint32_t AHEAD>
-__device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blocks, int stride, uint32_t* status) {
+// list build (passes 592 -> 520 us each, lists 1683 -> 1551 us).  finish(before, word, blocks), where a wait runs out, is a
+// call that ends the walk: with the counting inside the loop the rank sort of 30M tets took 1065 us in place of 897.
+template <uint32_t AHEAD, typename F>
+__device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blocks, int stride, F finish) {
   uint32_t before = 0;
   for (;;) {
     uint32_t v[AHEAD];
@@ -284,10 +315,7 @@ __device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blo
     for (uint32_t k = 0; k < AHEAD; ++k) {
       if (v[k] == 0u) {
         for (int polls = 0; v[k] == 0u && polls < kMaxPolls; ++polls) v[k] = load_relaxed(word - (int64_t)(k + 1) * stride);
-        if (v[k] == 0u) {
-          atomicOr(status, RM_STATUS_INTERNAL);
-          return before;
-        }
+        if (v[k] == 0u) return finish(before, word - (int64_t)k * stride, blocks - k);
       }
       if (v[k] & kRunEnd) return before + (v[k] ^ kRunEnd);
       before += v[k] - 1u;
@@ -298,16 +326,14 @@ __device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blo
 }
 
 // The same for one word per block, by a whole warp, 32 words at a time.
-__device__ __forceinline__ uint32_t warp_look_back(const uint32_t* word, uint32_t blocks, uint32_t* status) {
+template <typename F>
+__device__ __forceinline__ uint32_t warp_look_back(const uint32_t* word, uint32_t blocks, F finish) {
   const uint32_t lane = threadIdx.x & 31;
   uint32_t before = 0;
   for (;;) {
     uint32_t v = lane < blocks ? load_relaxed(word - lane - 1) : kRunEnd;
     for (int polls = 0; __any_sync(0xffffffffu, v == 0u); ++polls) {
-      if (polls == kMaxPolls) {
-        if (lane == 0) atomicOr(status, RM_STATUS_INTERNAL);
-        return before;
-      }
+      if (polls == kMaxPolls) return finish(before, word, blocks);
       if (v == 0u) v = load_relaxed(word - lane - 1);
     }
     const uint32_t ends = __ballot_sync(0xffffffffu, (v & kRunEnd) != 0u);
@@ -322,11 +348,11 @@ __device__ __forceinline__ uint32_t warp_look_back(const uint32_t* word, uint32_
 // Thread d (of 256) places the runs of digit d.  In: cnt[w][d], how many items of the digit warp w of this block holds,
 // and the digit's total over all blocks.  Out: cnt[w][d] the offset of the warp's items inside the block's run, lstart[d]
 // where the run starts in the block's reordered buffer, dbase[d] what to add to a position there for its global one.
-// Returns the number of items of the block.
-template <uint32_t AHEAD>
+// Returns the number of items of the block.  finish: see look_back.
+template <uint32_t AHEAD, typename F>
 __device__ __forceinline__ uint32_t place_runs(bool live, uint32_t digit_total, uint32_t tile, uint32_t* __restrict__ look,
                                                int bins, uint32_t* cnt, uint32_t* dbase, uint32_t* lstart, uint32_t* sm,
-                                               uint32_t* status) {
+                                               F finish) {
   const uint32_t d = threadIdx.x;
   uint32_t run = 0;
 #pragma unroll
@@ -341,12 +367,27 @@ __device__ __forceinline__ uint32_t place_runs(bool live, uint32_t digit_total, 
   const uint32_t ls = block_exclusive_scan<kSortThreads>(run, &n_block, sm);
   const uint32_t digit_base = block_exclusive_scan<kSortThreads>(digit_total, &unused, sm);
   if (live && tile > 0) {
-    before = look_back<AHEAD>(word, tile, bins, status);
+    before = look_back<AHEAD>(word, tile, bins, finish);
     store_relaxed(word, kRunEnd | (before + run));
   }
   lstart[d] = ls;
   dbase[d] = digit_base + before - ls;
   return n_block;
+}
+
+// finish_look_back of a pass of the rank sort whose blocks hold `tile` keys; a thread per digit.
+__device__ __noinline__ uint32_t count_digits_before(uint32_t before, const uint32_t* word, uint32_t blocks, const uint32_t* keys,
+                                                     int tile, int shift) {
+  note_recount(kRecountRankPass);
+  return finish_look_back(before, word, blocks, kRadix, [&](uint32_t b) {
+    uint32_t n = 0;
+#pragma unroll 1
+    for (int i = 0; i < tile; ++i) {
+      const uint32_t key = keys[(int64_t)b * tile + i];
+      n += key != kCulledKey && ((key >> shift) & (kRadix - 1)) == threadIdx.x;
+    }
+    return n;
+  });
 }
 
 // One stable pass.  The block's pairs are first reordered by digit in shared memory, so that the global stores of one
@@ -406,8 +447,11 @@ k_rank_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ v
     rnk[k] = prev + before;
   }
   __syncthreads();
-  const uint32_t n_block =
-      place_runs<2>(true, __ldg(hist + threadIdx.x), tile, look, kRadix, cnt, dbase, lstart, sm, &counters->status);
+  const uint32_t n_block = place_runs<2>(
+      true, __ldg(hist + threadIdx.x), tile, look, kRadix, cnt, dbase, lstart, sm,
+      [&](uint32_t before, const uint32_t* word, uint32_t blocks) {
+        return count_digits_before(before, word, blocks, keys_in, kSortTile, shift);
+      });
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kSortItems; ++k) {
@@ -424,6 +468,19 @@ k_rank_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ v
     if (pass < 3) keys_out[g] = pr.x;  // nobody reads the keys of the last pass
     vals_out[g] = pr.y;
   }
+}
+
+// finish_look_back of k_rank_rects, by a warp.
+__device__ __noinline__ uint32_t count_touched_before(uint32_t before, const uint32_t* word, uint32_t blocks,
+                                                      const uint32_t* order, const int4* rect) {
+  note_recount(kRecountRankRects);
+  // every lane may see another state of a word: the sum is lane 0's, which the count needs no lane to agree with
+  return __shfl_sync(0xffffffffu, finish_look_back(before, word, blocks, 1, [&](uint32_t b) {
+    uint32_t n = 0;
+#pragma unroll 1
+    for (int i = 0; i < kScanTile; ++i) n += regions_touched(rect[order[(int64_t)b * kScanTile + i]]);
+    return n & 0x3FFFFFFFu;
+  }), 0);
 }
 
 // Ranked rectangles: rect[order[i]] for every visible rank i, in rank order; the inclusive scan of the number of regions
@@ -470,7 +527,10 @@ k_rank_rects(const uint32_t* __restrict__ order, const int4* __restrict__ rect, 
   if (threadIdx.x < 32) {
     // more pairs than a list can hold are reported through n_keys: the words only must not lose their flags
     if (threadIdx.x == 0) store_relaxed(look + tile, tile == 0 ? kRunEnd | (total & ~kRunEnd) : (total & 0x3FFFFFFFu) + 1u);
-    const uint32_t before = tile ? warp_look_back(look + tile, tile, &counters->status) : 0u;
+    const uint32_t before =
+        tile == 0 ? 0u : warp_look_back(look + tile, tile, [&](uint32_t sum, const uint32_t* word, uint32_t blocks) {
+          return count_touched_before(sum, word, blocks, order, rect);
+        });
     if (threadIdx.x == 0) {
       if (tile) store_relaxed(look + tile, kRunEnd | ((before + total) & ~kRunEnd));
       s_before = before;
@@ -721,6 +781,18 @@ __device__ __noinline__ void layout_regions(const RegionTable& t) {
   }
 }
 
+// finish_look_back of k_region_pass; a thread per digit.
+__device__ __noinline__ uint32_t count_pairs_before(uint32_t before, const uint32_t* word, uint32_t blocks, const uint2* pairs,
+                                                    int tile, int shift, uint32_t bins) {
+  note_recount(kRecountRegionPass);
+  return finish_look_back(before, word, blocks, (int)bins, [&](uint32_t b) {
+    uint32_t n = 0;
+#pragma unroll 1
+    for (int i = 0; i < tile; ++i) n += ((pairs[(int64_t)b * tile + i].y >> shift) & (bins - 1)) == threadIdx.x;
+    return n;
+  });
+}
+
 // One stable pass on the digit (code >> shift) & (2^BITS - 1).  final == 0: the reordered pairs go to pairs_out;
 // final != 0: the sorted entries (tet id, tile mask) are written instead, and the regions' entries are counted: in the
 // block's reordered buffer a region's pairs are contiguous, so that the position of a run's first pair is subtracted
@@ -729,7 +801,7 @@ template <int BITS, int kBinItems>
 __global__ void __launch_bounds__(kBinThreads, 3)
 k_region_pass(const uint2* __restrict__ pairs, int64_t n, int shift, const uint32_t* __restrict__ digit_total,
               uint32_t* __restrict__ ticket, uint32_t* __restrict__ look /* [blocks][2^BITS], zeroed */,
-              uint32_t* __restrict__ status, int final, uint2* __restrict__ pairs_out, uint2* __restrict__ entries,
+              int final, uint2* __restrict__ pairs_out, uint2* __restrict__ entries,
               RegionTable table) {
   after_previous();
   constexpr int kBinTile = kBinThreads * kBinItems;
@@ -780,7 +852,9 @@ k_region_pass(const uint2* __restrict__ pairs, int64_t n, int shift, const uint3
   }
   __syncthreads();
   place_runs<8>(threadIdx.x < bins, threadIdx.x < bins ? __ldg(digit_total + threadIdx.x) : 0u, tile, look, (int)bins, cnt, dbase,
-             lstart, sm, status);
+                lstart, sm, [&](uint32_t before, const uint32_t* word, uint32_t blocks) {
+                  return count_pairs_before(before, word, blocks, pairs, kBinTile, shift, bins);
+                });
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kBinItems; ++k) {
@@ -861,11 +935,22 @@ __device__ __forceinline__ uint32_t region_of_chunk(const uint32_t* __restrict__
 constexpr int kFineRounds = kChunk / 32;
 constexpr int kFineStride = kChunk + 4;  // bytes per tile: the lanes' byte stores fall into different banks
 
+// finish_look_back of k_fine_lists over the chunks of a region, whose entries start at `first`; a lane per tile.
+__device__ __noinline__ uint32_t count_covering_before(uint32_t before, const uint32_t* word, uint32_t chunks, const uint2* first) {
+  note_recount(kRecountFineLists);
+  return finish_look_back(before, word, chunks, 32, [&](uint32_t k) {
+    uint32_t n = 0;
+#pragma unroll 1
+    for (int i = 0; i < kChunk; ++i) n += (first[(int64_t)k * kChunk + i].y >> (threadIdx.x & 31)) & 1u;
+    return n;
+  });
+}
+
 __global__ void __launch_bounds__(kFineThreads)
 k_fine_lists(const uint2* __restrict__ entries, const uint32_t* __restrict__ region_start,
              const uint32_t* __restrict__ chunk_base, uint32_t n_regions, int reg_w, int grid_w, int grid_h,
              const uint32_t* __restrict__ tile_start, uint32_t* __restrict__ ticket, uint32_t* __restrict__ look /* zeroed */,
-             uint32_t* __restrict__ status, uint32_t* __restrict__ digit_total, uint32_t n_keys,
+             uint32_t* __restrict__ digit_total, uint32_t n_keys,
              int32_t* __restrict__ sorted_idx) {
   after_previous();
   __shared__ uint8_t s_pos[kFineWarps][32 * kFineStride];
@@ -913,7 +998,9 @@ k_fine_lists(const uint2* __restrict__ entries, const uint32_t* __restrict__ reg
   }
   uint32_t before = 0;
   if (k_in_region) {
-    before = look_back<8>(mine, k_in_region, 32, status);
+    before = look_back<8>(mine, k_in_region, 32, [&](uint32_t sum, const uint32_t* word, uint32_t chunks) {
+      return count_covering_before(sum, word, chunks, entries + (begin - k_in_region * kChunk));
+    });
     store_relaxed(mine, kRunEnd | (before + n));
   }
   const int gy = (int)(r / (uint32_t)reg_w), gx = (int)(r - (uint32_t)gy * (uint32_t)reg_w);
@@ -1187,7 +1274,7 @@ int rm_launch_build_lists(const int32_t* rect, const int32_t* tile_ranges, int64
       auto kernel = P.items == 4 ? pass_kernel<4>(P.bits) : pass_kernel<16>(P.bits);
       RM_CUDA_CHECK(rm_launch_behind(n_region_keys, kernel, (unsigned)P.nblk, rm::kBinThreads, 0, st, pairs[pass & 1],
                                      n_region_keys, rm::kCodeBits + pass * P.bits, digit_total + pass * rm::kRadix,
-                                     tickets + pass, look, &counters->status, pass == P.passes - 1, pairs[(pass & 1) ^ 1],
+                                     tickets + pass, look, pass == P.passes - 1, pairs[(pass & 1) ^ 1],
                                      entries, table));
     }
   }
@@ -1195,10 +1282,22 @@ int rm_launch_build_lists(const int32_t* rect, const int32_t* tile_ranges, int64
     RmProfScope prof("k_fine_lists", st);
     RM_CUDA_CHECK(rm_launch_behind(n_region_keys, rm::k_fine_lists, (unsigned)((P.max_chunks + rm::kFineWarps - 1) / rm::kFineWarps),
                                    rm::kFineThreads, 0, st, entries, table.start, table.chunk_base, P.n_regions, P.reg_w, gw, gh,
-                                   tile_start, tickets + rm::kMaxPasses, fine_look, &counters->status, digit_total,
+                                   tile_start, tickets + rm::kMaxPasses, fine_look, digit_total,
                                    (uint32_t)n_keys, sorted_idx));
   }
   return RM_OK;
 }
 
 unsigned rm_bounds_status_binning() { return rm_take_bounds_status(); }
+
+// Checked build: which kinds of look-back words have been counted by waiting blocks since the last call, else 0.
+unsigned rm_take_recounted() {
+  unsigned v = 0;
+#ifdef RM_BOUNDS_CHECK
+  const unsigned z = 0;
+  cudaDeviceSynchronize();
+  cudaMemcpyFromSymbol(&v, rm::g_recounted, sizeof(v));
+  cudaMemcpyToSymbol(rm::g_recounted, &z, sizeof(z));
+#endif
+  return v;
+}

@@ -120,6 +120,7 @@ static inline unsigned rm_take_bounds_status() { return 0; }
 #endif
 unsigned rm_bounds_status_raster();
 unsigned rm_bounds_status_binning();
+unsigned rm_take_recounted();
 
 namespace rm {
 

@@ -71,8 +71,6 @@ def read_info(ctx):
         raise AssertionError("Tensor contains NaN values!")
     if status & _lib.RM_STATUS_BAD_INDEX:
         raise IndexError("rm_b200: indices name a vertex outside [0, n_vertices)")
-    if status & _lib.RM_STATUS_INTERNAL:
-        raise RuntimeError("rm_b200: the rank sort did not complete")
     if status & _lib.RM_STATUS_KEY_OVERFLOW or n_keys > 2**31 - 1:
         raise RuntimeError(f"rm_b200: {n_keys} (tile, tet) pairs exceed the int32 range of the tile lists")
     return n_keys, n_visible
