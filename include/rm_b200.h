@@ -385,8 +385,8 @@ int64_t rm_launch_count(void);
  *   rm_debug_bounds_status: waits for the device, returns the status word and clears it (bit = access
  *     site; 0 = every checked access was inside its array).
  *   rm_debug_recounted: waits for the device, returns and clears one bit for each kind of look-back word (1 rank
- *     sort, 2 scan in rank order, 4 region sort, 8 tile lists) that a block has counted itself, which this build
- *     does whenever a word is not there at first sight (the ordinary one after some 10 ms of waiting).
+ *     sort, 2 scan in rank order, 4 region sort, 8 tile lists) that a block has counted itself; the ordinary build
+ *     does so after some 10 ms of waiting, this one always for the words of every other block.
  */
 int rm_debug_bounds_checked(void);
 void rm_debug_set_extent(int which, int64_t n);

@@ -230,7 +230,7 @@ constexpr uint32_t kCulledKey = 0xFFFFFFFFu;
 // itself, from the other blocks' items, which nothing writes while the kernel runs (finish_look_back).
 constexpr uint32_t kRunEnd = 1u << 31;
 #ifdef RM_BOUNDS_CHECK
-constexpr int kMaxPolls = 0;  // the checked build counts every word that is not there at first sight
+constexpr int kMaxPolls = 0;  // the checked build waits for no word, and never sees those of every other block (look_word)
 static __device__ unsigned g_recounted;
 #else
 constexpr int kMaxPolls = 1 << 14;  // about 10 ms per word
@@ -284,6 +284,15 @@ __device__ __forceinline__ void store_relaxed(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v));
 }
 
+__device__ __forceinline__ uint32_t look_word(const uint32_t* p, uint32_t block) {
+#ifdef RM_BOUNDS_CHECK
+  if (block & 1u) return 0u;
+#else
+  (void)block;
+#endif
+  return load_relaxed(p);
+}
+
 // Sum of what the `blocks` blocks before `word` hold, on top of `before`, without waiting; count(b): what block b holds.
 template <typename F>
 __device__ __forceinline__ uint32_t finish_look_back(uint32_t before, const uint32_t* word, uint32_t blocks, int stride, F count) {
@@ -291,7 +300,7 @@ __device__ __forceinline__ uint32_t finish_look_back(uint32_t before, const uint
   while (blocks) {
     --blocks;
     word -= stride;
-    uint32_t v = load_relaxed(word);
+    uint32_t v = look_word(word, blocks);
     if (v == 0u) v = count(blocks) + 1u;
     if (v & kRunEnd) return before + (v ^ kRunEnd);
     before += v - 1u;
@@ -310,7 +319,7 @@ __device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blo
   for (;;) {
     uint32_t v[AHEAD];
 #pragma unroll
-    for (uint32_t k = 0; k < AHEAD; ++k) v[k] = k < blocks ? load_relaxed(word - (int64_t)(k + 1) * stride) : kRunEnd;
+    for (uint32_t k = 0; k < AHEAD; ++k) v[k] = k < blocks ? look_word(word - (int64_t)(k + 1) * stride, blocks - 1u - k) : kRunEnd;
 #pragma unroll
     for (uint32_t k = 0; k < AHEAD; ++k) {
       if (v[k] == 0u) {
@@ -331,7 +340,7 @@ __device__ __forceinline__ uint32_t warp_look_back(const uint32_t* word, uint32_
   const uint32_t lane = threadIdx.x & 31;
   uint32_t before = 0;
   for (;;) {
-    uint32_t v = lane < blocks ? load_relaxed(word - lane - 1) : kRunEnd;
+    uint32_t v = lane < blocks ? look_word(word - lane - 1, blocks - 1u - lane) : kRunEnd;
     for (int polls = 0; __any_sync(0xffffffffu, v == 0u); ++polls) {
       if (polls == kMaxPolls) return finish(before, word, blocks);
       if (v == 0u) v = load_relaxed(word - lane - 1);

@@ -1,6 +1,6 @@
-"""Waits of the sorts that run out: in the checked build a block that finds a look-back word missing does not wait for it but
-counts the other block's items itself, as the ordinary build does after some milliseconds.  The lists have to be the
-oracle's all the same."""
+"""Waits of the sorts that run out: in the checked build a block waits for no look-back word and never sees those of every
+other block; it counts what is missing itself, as the ordinary build does after some milliseconds.  The lists have to be
+the oracle's all the same."""
 import os
 import subprocess
 import sys
