@@ -38,8 +38,8 @@ __device__ __forceinline__ uint32_t regions_touched(int4 rc) {
 }
 
 // number of valid items: n, or the device-side count if one is given (the visible tets, known only on the device)
-__device__ __forceinline__ int64_t valid_items(int64_t n, const uint32_t* __restrict__ n_dev) {
-  return n_dev ? min(n, (int64_t)__ldg(n_dev)) : n;
+__device__ __forceinline__ int64_t valid_items(int64_t n, const uint32_t* n_dev) {
+  return n_dev ? min(n, (int64_t)*n_dev) : n;
 }
 
 // Counters of one call, zeroed with the tile-coverage arrays before the projection.
@@ -87,11 +87,11 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
 }
 
 // sum of the block sums before this block's, and, if `total` is given, of all n of them (else n is this block's index)
-__device__ __forceinline__ uint32_t sums_before(const uint32_t* __restrict__ bsum, uint32_t n, unsigned long long* total) {
+__device__ __forceinline__ uint32_t sums_before(const uint32_t* bsum, uint32_t n, unsigned long long* total) {
   __shared__ unsigned long long before[kScanThreads / 32], all[kScanThreads / 32];
   unsigned long long b = 0, t = 0;
   for (uint32_t i = threadIdx.x; i < n; i += kScanThreads) {
-    const uint32_t v = __ldg(bsum + i);
+    const uint32_t v = bsum[i];
     if (i < blockIdx.x) b += v;
     t += v;
   }
@@ -116,7 +116,7 @@ __device__ __forceinline__ uint32_t sums_before(const uint32_t* __restrict__ bsu
 }
 
 // blocked arrangement: thread t owns items [t*kScanItems, (t+1)*kScanItems) of its block
-__device__ __forceinline__ void load_blocked(const uint32_t* __restrict__ in, int64_t base, int64_t n, uint32_t (&v)[kScanItems]) {
+__device__ __forceinline__ void load_blocked(const uint32_t* in, int64_t base, int64_t n, uint32_t (&v)[kScanItems]) {
   if (base + kScanItems <= n) {
 #pragma unroll
     for (int k = 0; k < kScanItems; k += 4) {
@@ -245,7 +245,7 @@ __device__ __forceinline__ void note_recount(Recounted which) {
 }
 
 __global__ void __launch_bounds__(kSortThreads)
-k_digit_hist(const uint32_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist /* [4][kRadix], zeroed */, TileJob job) {
+k_digit_hist(const uint32_t* keys, int64_t n, uint32_t* __restrict__ hist /* [4][kRadix], zeroed */, TileJob job) {
   after_previous();
   constexpr int kItems = 8, kTile = kItems * kSortThreads;
   if ((int)blockIdx.x < job.blocks) return run_tile_job(job);
@@ -259,7 +259,7 @@ k_digit_hist(const uint32_t* __restrict__ keys, int64_t n, uint32_t* __restrict_
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
       const int64_t i = base + k * kSortThreads + threadIdx.x;
-      key[k] = i < n ? __ldg(keys + i) : kCulledKey;
+      key[k] = i < n ? keys[i] : kCulledKey;
     }
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
@@ -403,8 +403,8 @@ __device__ __noinline__ uint32_t count_digits_before(uint32_t before, const uint
 // digit's run are contiguous.  FIRST: the tet of item i is i.
 template <bool FIRST, int kSortItems>
 __global__ void __launch_bounds__(kSortThreads, 3)
-k_rank_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, int64_t T, BinCounters* __restrict__ counters,
-            int pass, const uint32_t* __restrict__ hist, uint32_t* __restrict__ look /* [blocks][kRadix], zeroed */,
+k_rank_pass(const uint32_t* keys_in, const uint32_t* vals_in, int64_t T, BinCounters* counters, int pass,
+            const uint32_t* hist, uint32_t* __restrict__ look /* [blocks][kRadix], zeroed */,
             uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, TileJob job) {
   after_previous();
   constexpr int kSortTile = kSortThreads * kSortItems;
@@ -457,7 +457,7 @@ k_rank_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ v
   }
   __syncthreads();
   const uint32_t n_block = place_runs<2>(
-      true, __ldg(hist + threadIdx.x), tile, look, kRadix, cnt, dbase, lstart, sm,
+      true, hist[threadIdx.x], tile, look, kRadix, cnt, dbase, lstart, sm,
       [&](uint32_t before, const uint32_t* word, uint32_t blocks) {
         return count_digits_before(before, word, blocks, keys_in, kSortTile, shift);
       });
@@ -497,7 +497,7 @@ __device__ __noinline__ uint32_t count_touched_before(uint32_t before, const uin
 // gathering them once, here, is a fraction of the three gathers per pair that it took to read them by tet id.  One launch
 // with look-back: the counts change hands in shared memory between the gather's striped order and the scan's blocked one.
 __global__ void __launch_bounds__(kScanThreads)
-k_rank_rects(const uint32_t* __restrict__ order, const int4* __restrict__ rect, int64_t T, BinCounters* __restrict__ counters,
+k_rank_rects(const uint32_t* order, const int4* rect, int64_t T, BinCounters* counters,
              uint32_t* __restrict__ look /* zeroed */, int4* __restrict__ ranked, uint32_t* __restrict__ cum,
              RmBinInfo* __restrict__ info, RmBinInfo* __restrict__ host_info) {
   after_previous();
@@ -522,7 +522,7 @@ k_rank_rects(const uint32_t* __restrict__ order, const int4* __restrict__ rect, 
     const int j = k * kScanThreads + threadIdx.x;
     uint32_t v = 0;
     if (first + j < n && RM_INDEX_OK(id[k], RM_X_TETS, 13)) {
-      const int4 rc = __ldg(rect + id[k]);
+      const int4 rc = rect[id[k]];
       ranked[first + j] = rc;
       v = regions_touched(rc);
     }
@@ -808,7 +808,7 @@ __device__ __noinline__ uint32_t count_pairs_before(uint32_t before, const uint3
 // from its region's count and the position behind its last added.
 template <int BITS, int kBinItems>
 __global__ void __launch_bounds__(kBinThreads, 3)
-k_region_pass(const uint2* __restrict__ pairs, int64_t n, int shift, const uint32_t* __restrict__ digit_total,
+k_region_pass(const uint2* pairs, int64_t n, int shift, const uint32_t* digit_total,
               uint32_t* __restrict__ ticket, uint32_t* __restrict__ look /* [blocks][2^BITS], zeroed */,
               int final, uint2* __restrict__ pairs_out, uint2* __restrict__ entries,
               RegionTable table) {
@@ -834,7 +834,7 @@ k_region_pass(const uint2* __restrict__ pairs, int64_t n, int shift, const uint3
 #pragma unroll
   for (int k = 0; k < kBinItems; ++k) {
     const int jl = warp * kBinSpan + k * 32 + lane;
-    pr[k] = jl < n_block ? __ldg(pairs + base + jl) : make_uint2(0u, 0u);
+    pr[k] = jl < n_block ? pairs[base + jl] : make_uint2(0u, 0u);
   }
   uint32_t rnk[kBinItems / 2];
 #pragma unroll
@@ -860,7 +860,7 @@ k_region_pass(const uint2* __restrict__ pairs, int64_t n, int shift, const uint3
     if (k & 1) rnk[k >> 1] |= r << 16; else rnk[k >> 1] = r;
   }
   __syncthreads();
-  place_runs<8>(threadIdx.x < bins, threadIdx.x < bins ? __ldg(digit_total + threadIdx.x) : 0u, tile, look, (int)bins, cnt, dbase,
+  place_runs<8>(threadIdx.x < bins, threadIdx.x < bins ? digit_total[threadIdx.x] : 0u, tile, look, (int)bins, cnt, dbase,
                 lstart, sm, [&](uint32_t before, const uint32_t* word, uint32_t blocks) {
                   return count_pairs_before(before, word, blocks, pairs, kBinTile, shift, bins);
                 });
@@ -918,12 +918,12 @@ __device__ __forceinline__ uint32_t warp_bit_transpose(uint32_t a) {
 }
 
 // Region of a chunk: the last r with chunk_base[r] <= chunk, found by the whole warp, 32 probes a round.
-__device__ __forceinline__ uint32_t region_of_chunk(const uint32_t* __restrict__ chunk_base, uint32_t n_regions, uint32_t chunk) {
+__device__ __forceinline__ uint32_t region_of_chunk(const uint32_t* chunk_base, uint32_t n_regions, uint32_t chunk) {
   uint32_t lo = 0, hi = n_regions;  // first index with chunk_base > chunk lies in [lo, hi]: chunk_base[n_regions] > chunk
   while (lo < hi) {
     const uint32_t step = (hi - lo + 31) / 32;
     const uint32_t probe = min(lo + ((threadIdx.x & 31) + 1) * step, hi) - 1;
-    const uint32_t c = __popc(__ballot_sync(0xffffffffu, __ldg(chunk_base + probe) <= chunk));
+    const uint32_t c = __popc(__ballot_sync(0xffffffffu, chunk_base[probe] <= chunk));
     if (c == 32) {
       lo = hi;
     } else {
@@ -956,10 +956,9 @@ __device__ __noinline__ uint32_t count_covering_before(uint32_t before, const ui
 }
 
 __global__ void __launch_bounds__(kFineThreads)
-k_fine_lists(const uint2* __restrict__ entries, const uint32_t* __restrict__ region_start,
-             const uint32_t* __restrict__ chunk_base, uint32_t n_regions, int reg_w, int grid_w, int grid_h,
-             const uint32_t* __restrict__ tile_start, uint32_t* __restrict__ ticket, uint32_t* __restrict__ look /* zeroed */,
-             uint32_t* __restrict__ digit_total, uint32_t n_keys,
+k_fine_lists(const uint2* entries, const uint32_t* region_start, const uint32_t* chunk_base, uint32_t n_regions, int reg_w,
+             int grid_w, int grid_h, const uint32_t* __restrict__ tile_start, uint32_t* __restrict__ ticket,
+             uint32_t* __restrict__ look /* zeroed */, uint32_t* __restrict__ digit_total, uint32_t n_keys,
              int32_t* __restrict__ sorted_idx) {
   after_previous();
   __shared__ uint8_t s_pos[kFineWarps][32 * kFineStride];
@@ -971,12 +970,12 @@ k_fine_lists(const uint2* __restrict__ entries, const uint32_t* __restrict__ reg
   if (s_block == 0)  // nobody needs them any more; the lists can then be built again from the same first half
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kFineThreads) digit_total[i] = 0;
   const uint32_t chunk = s_block * kFineWarps + warp;
-  if (chunk >= __ldg(chunk_base + n_regions)) return;
+  if (chunk >= chunk_base[n_regions]) return;
   if (!RM_INDEX_OK(chunk, RM_X_CHUNKS, 10)) return;
   const uint32_t r = region_of_chunk(chunk_base, n_regions, chunk);
-  const uint32_t k_in_region = chunk - __ldg(chunk_base + r);
-  const uint32_t begin = __ldg(region_start + r) + k_in_region * kChunk;
-  const uint32_t count = min((uint32_t)kChunk, __ldg(region_start + r + 1) - begin);
+  const uint32_t k_in_region = chunk - chunk_base[r];
+  const uint32_t begin = region_start[r] + k_in_region * kChunk;
+  const uint32_t count = min((uint32_t)kChunk, region_start[r + 1] - begin);
   uint8_t* pos = s_pos[warp] + lane * kFineStride;
   int32_t* ids = s_id[warp];
   uint32_t word[kFineRounds], n = 0;
@@ -985,7 +984,7 @@ k_fine_lists(const uint2* __restrict__ entries, const uint32_t* __restrict__ reg
 #pragma unroll
     for (int k = 0; k < kFineRounds; ++k) {
       const uint32_t e = 32 * k + lane;
-      en[k] = (e < count && RM_INDEX_OK(begin + e, RM_X_PAIRS, 9)) ? __ldg(entries + begin + e) : make_uint2(0u, 0u);
+      en[k] = (e < count && RM_INDEX_OK(begin + e, RM_X_PAIRS, 9)) ? entries[begin + e] : make_uint2(0u, 0u);
     }
 #pragma unroll
     for (int k = 0; k < kFineRounds; ++k) {

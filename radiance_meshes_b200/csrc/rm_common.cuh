@@ -124,9 +124,13 @@ unsigned rm_take_recounted();
 
 namespace rm {
 
-// First statement of every thread of a kernel that may be launched with rm_launch_behind, before any access to memory: lets
-// the next kernel's blocks be placed as soon as all of this one's are, and waits until the kernel before has ended and what
-// it wrote can be seen.  Returns at once after an ordinary launch.
+// First statement of every thread of a kernel that may be launched with rm_launch_behind, or in front of one, before any
+// access to memory: lets the next kernel's blocks be placed as soon as all of this one's are, and waits until the kernel
+// before has ended and what it wrote can be seen.  The wait returns at once after an ordinary launch.
+// A kernel that is launched behind another is there while the kernels before it in the chain still write.  What those
+// write it reads with plain loads from pointers without __restrict__: __ldg, and const __restrict__, tell the compiler that
+// the data stay the same for as long as the kernel is there, which lets it move the loads in front of the wait and serve
+// them from a cache that is not kept coherent.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");

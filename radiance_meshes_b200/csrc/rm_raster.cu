@@ -1687,7 +1687,7 @@ k_distortion_loss(const float* __restrict__ dist, int64_t n, float* __restrict__
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 __global__ void __launch_bounds__(kLossThreads)
-k_distortion_loss_mean(const float* __restrict__ partials, int n_partials, int64_t n, float* __restrict__ loss) {
+k_distortion_loss_mean(const float* partials, int n_partials, int64_t n, float* __restrict__ loss) {
   after_previous();
   float sum = 0.0f;
   for (int i = threadIdx.x; i < n_partials; i += kLossThreads) sum += partials[i];
