@@ -24,7 +24,7 @@ __device__ __forceinline__ float safe_div_torch(float n, float d) {
 
 __device__ __forceinline__ void act_cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ float sh_load(const float* p) { return *p; }
 __device__ __forceinline__ float sh_load(const __half* p) { return __half2float(*p); }
@@ -55,7 +55,7 @@ k_activate_output(const float* __restrict__ camera_center, const float* __restri
     } else {
       for (int i = threadIdx.x; i < rows * row_vals; i += kActThreads) sh_s[i] = src[i];
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
   const int64_t g = first + threadIdx.x;
   const bool live = g < T;
@@ -92,7 +92,7 @@ k_activate_output(const float* __restrict__ camera_center, const float* __restri
     }
   }
   if (deg > 0) {
-    asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
   }
   if (live) {

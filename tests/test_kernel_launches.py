@@ -75,3 +75,12 @@ def test_kernels_behind_others_do_not_read_what_those_write_as_constant_data():
     behind = re.findall(r"rm_launch_behind\([^;]*?(k_\w+)", " ".join(texts.values()))
     assert {"k_rank_rects", "k_digit_hist", "k_fine_lists", "k_distortion_loss_mean"} <= set(behind)
     assert set(behind) <= seen and {"k_rank_pass", "k_region_pass", "k_backward", "k_project_deferred"} <= seen
+
+
+def test_asynchronous_copies_are_ordered_for_the_compiler():
+    """An asm statement with a "memory" clobber is a place that no access to memory moves across."""
+    found = [s for text in sources().values() for s in re.findall(r'asm volatile\((?:"[^"]*"|[^";])*;', text)
+             if "cp.async" in s or "griddepcontrol" in s]
+    assert len(found) >= 6
+    for statement in found:
+        assert '"memory"' in statement, statement
