@@ -181,7 +181,8 @@ int rm_forward(const int32_t* sorted_tetra_idx, const int32_t* tile_ranges, cons
                int32_t* n_contributors, const RmHitList* hits, void* stream);
 /*
  * The same for a caller that knows n_list, the number of entries of all tile lists: large images then start with the tiles
- * whose lists are long against the average.
+ * whose lists are long against the average.  The outputs of both have the same bits, and so has a row of the image in calls
+ * for different bands.
  */
 int rm_forward_sized(const int32_t* sorted_tetra_idx, const int32_t* tile_ranges, const float* records,
                      const RmCamera* cam, const float* ray_jitter, float* output_img, float* distortion_img,

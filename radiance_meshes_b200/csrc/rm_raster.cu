@@ -415,7 +415,7 @@ __device__ __forceinline__ bool slab_test(const float4 (&rec)[4], const Ray& d, 
   e.enter = fmaxf(e.te, 0.0f);
   e.exit = h.ux - min_t;
   e.dt = e.exit - e.enter;
-  e.tau = density * e.dt;
+  e.tau = __fmul_rn(density, e.dt);  // never fused into the sum of optical depths
   return e.tau > 0.0f;
 }
 
@@ -455,17 +455,18 @@ __device__ __forceinline__ void segment_weights(float x, float& alpha, float& w0
   // p = 1/2 - x/6 + x^2/24 - x^3/120 + x^4/720 - x^5/5040
   const float p = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 5040.0f, 1.0f / 720.0f), -1.0f / 120.0f), 1.0f / 24.0f),
                                -1.0f / 6.0f), 0.5f);
-  const float inv = fast_rcp(x), phi = (1.0f - alpha) * inv;
+  const float inv = fast_rcp(x), rest = 1.0f - alpha, series = __fmul_rn(x, p);
   // both forms are evaluated: the lanes of a warp nearly always need both, and selects cost less than the branch
   const bool thin = x < 0.25f;
-  w1 = thin ? x * p : 1.0f - phi;
-  w0 = thin ? fmaf(-x, w1, x) - w1 : phi - alpha;
+  w1 = thin ? series : fmaf(-rest, inv, 1.0f);
+  w0 = thin ? fmaf(-x, series, x) - series : fmaf(rest, inv, -alpha);
   slope = thin ? (1.0f - w1) - p : w0 * inv;
 }
 
-// colour of the segment of a hit
+// Colour of the segment of a hit.  Here and in what it calls the contraction is spelled out, so that every walk that the
+// compiler builds from it has the same bits.
 __device__ __forceinline__ void integrate(float4 cg, float4 cb, f3 d, float min_t, Eval& e) {
-  const float gd = cg.x * d.x + cg.y * d.y + cg.z * d.z;
+  const float gd = dot_fma({cg.x, cg.y, cg.z}, d);
   const float oe = fmaf(e.enter + min_t, gd, cg.w), ox = fmaf(e.exit + min_t, gd, cg.w);
   float w0, w1, slope;
   segment_weights(e.tau, e.alpha, w0, w1, slope);
@@ -665,9 +666,9 @@ struct StatsArgs {
 };
 // How the units of 16 pixels are dealt to warps; the rule is at rm_launch_forward.
 //   halves:     two units per warp, one per half: every lane walks its pixel's entries one by one.
-//   pairs:      one unit per warp, and two lanes per pixel: each evaluates every other entry that covers the pixel, and the
-//               optical depths and moments of the two change hands by shuffles, so that the state goes through the entries
-//               in list order all the same.  Steps and batches of 32 entries in place of 16.  Half the serial chain per
+//   pairs:      one unit per warp, and two lanes per pixel: each evaluates every other entry that covers the pixel, and
+//               what the second has found goes to the first by shuffles, which takes the two through the pixel's state in
+//               list order.  Steps and batches of 32 entries in place of 16.  Half the serial chain per
 //               unit, which is what a grid that fills the chip once or a few times waits for, for 12 % more issue and
 //               shared-memory work per hit (128 x 128 pixels, 13k tets: 54 -> 37 us; 720 x 720 fisheye, 1M tets:
 //               414 -> 291 us; 822 x 1237, 2M tets, evenly long lists: 1.87 -> 2.08 ms;
@@ -675,8 +676,32 @@ struct StatsArgs {
 //   long first: tiles with long lists first, by pairs, the rest by halves.  A unit of 3,000 candidates among units of 100
 //               otherwise starts when its turn in the raster comes, and the chip waits for it at the end (6M tets, 1080p:
 //               1.88 -> 1.64 ms; 18M: 3.27 -> 2.49 ms).
+// A pixel's hits are taken in the same order with the same operations in all of them: which one a call uses cannot be told
+// from the bits of its image, so that a frame in bands, each dealt by its own size, is the frame.
 // Slot of (entry, pixel): the exclusive-or spreads the accesses by pixel and by entry over the banks.
 __device__ __forceinline__ int entry_slot(int e, int p) { return e * 16 + (p ^ e); }
+
+// A pixel's state behind a hit: transmittance and distortion moments (dy without a factor of two, dv without one of a third).
+// m2: twice the first moment of the density over the segment; of the constant-colour variant the laddered distance.
+template <ForwardMode MODE>
+__device__ __forceinline__ void update_state(float tau, float alpha, float dens, float m2, float& T, float& logT, float& dx,
+                                             float& dy, float& dz, float& dw, float& dv) {
+  if (MODE == kConstColor) {
+    const float weight = __fmul_rn(T, 1.0f - alpha);
+    dx = fmaf(2.0f * weight * m2, dz, dx);
+    dy = fmaf(weight, dw, dy);
+    dz += weight;
+    dw = fmaf(weight, m2, dw);
+  } else {
+    logT -= tau;
+    dx = fmaf(m2, dz, dx);
+    dy = fmaf(dens, dw, dy);
+    dz += dens;
+    dw = fmaf(m2, 0.5f, dw);
+    dv = fmaf(dens, tau, dv);
+  }
+  T *= alpha;
+}
 
 template <ForwardMode MODE>
 using ForwardShared = typename std::conditional<MODE == kStats, StatsShared, FwdShared>::type;
@@ -886,61 +911,34 @@ __device__ __forceinline__ void walk_unit(
             missed |= bit;
           }
         }
-        // the pixel ends at the later entry, or (`early`) already at the earlier one
-        auto finish = [&](bool early) {
-          const int last = __shfl_sync(0x10001u << lane16, j, early ? lane16 : lane16 + 16);
-          active = false;
-          contrib = batch_pos[last] + 1;  // entries walked, the terminating one included
-          hitbits &= ~(0x7FFFFFFFu >> last);
-          mine = 0;
+        // The first lane of a pixel takes its two entries in list order, with the operations of the walk by halves: the bits of
+        // an image do not depend on how its units are dealt.  (The second lane goes along; its state is not used.)
+        const float o_tau = __shfl_xor_sync(FULL, e.tau, 16), o_alpha = __shfl_xor_sync(FULL, e.alpha, 16);
+        const float o_dens = __shfl_xor_sync(FULL, dens, 16), o_m2 = __shfl_xor_sync(FULL, m2, 16);
+        const float o_r = __shfl_xor_sync(FULL, e.cr, 16), o_g = __shfl_xor_sync(FULL, e.cg, 16);
+        const float o_b = __shfl_xor_sync(FULL, e.cb, 16);
+        // An entry that the pixel misses adds zeros, which costs less than a branch (60k tets, 203 x 317: 103 us, with branches
+        // 115); it changes nothing as long as no moment has overflowed.
+        auto take = [&](float tau, float alpha, float dens, float m2, float r, float g, float b) {
+          sr = fmaf(r, T, sr);
+          sg = fmaf(g, T, sg);
+          sb = fmaf(b, T, sb);
+          update_state<MODE>(tau, alpha, dens, m2, T, logT, dx, dy, dz, dw, dv);
+          return MODE == kConstColor ? T < 1.0f / 255.0f : logT < -5.5f;
         };
-        if constexpr (MODE == kConstColor) {
-          const float o_alpha = __shfl_xor_sync(FULL, e.alpha, 16), o_m = __shfl_xor_sync(FULL, m2, 16);
-          const float a1 = second ? o_alpha : e.alpha, a2 = second ? e.alpha : o_alpha;
-          const float T1 = T * a1, w1 = T * (1.0f - a1), before = second ? T1 : T;
-          float T2 = T1 * a2, w2 = T1 * (1.0f - a2);
-          if (T2 < 1.0f / 255.0f && active) {
-            const bool early = T1 < 1.0f / 255.0f;
-            finish(early);
-            if (early) {
-              T2 = T1;
-              w2 = 0.f;
-              if (second) e.cr = e.cg = e.cb = 0.f;
-            }
+        const bool early = take(e.tau, e.alpha, dens, m2, e.cr, e.cg, e.cb);
+        const bool late = take(early ? 0.0f : o_tau, early ? 1.0f : o_alpha, early ? 0.0f : o_dens, early ? 0.0f : o_m2,
+                               early ? 0.0f : o_r, early ? 0.0f : o_g, early ? 0.0f : o_b);
+        const unsigned ended = __ballot_sync(FULL, active && !second && late);
+        if (ended) {
+          const int at = __shfl_sync(FULL, (int)early, lane16) ? lane16 : lane16 + 16;
+          const int last = __shfl_sync(FULL, j, at);  // the entry at which the pixel has ended
+          if ((ended >> lane16) & 1u) {
+            active = false;
+            contrib = batch_pos[last] + 1;  // entries walked, the terminating one included
+            hitbits &= ~(0x7FFFFFFFu >> last);
+            mine = 0;
           }
-          sr = fmaf(e.cr, before, sr);
-          sg = fmaf(e.cg, before, sg);
-          sb = fmaf(e.cb, before, sb);
-          const float dz1 = dz + w1, dw1 = fmaf(w1, second ? o_m : m2, dw), w = second ? w2 : w1;
-          dx = fmaf(2.0f * w * m2, second ? dz1 : dz, dx);
-          dy = fmaf(w, second ? dw1 : dw, dy);
-          dz = dz1 + w2;
-          dw = fmaf(w2, second ? m2 : o_m, dw1);
-          T = T2;
-        } else {
-          const float o_tau = __shfl_xor_sync(FULL, e.tau, 16);
-          float o_dens = __shfl_xor_sync(FULL, dens, 16), o_m2 = __shfl_xor_sync(FULL, m2, 16);
-          const float logT1 = logT - (second ? o_tau : e.tau), logT2 = logT1 - (second ? e.tau : o_tau);
-          const float before = fast_exp(second ? logT1 : logT);
-          logT = logT2;
-          if (logT2 < -5.5f && active) {
-            const bool early = logT1 < -5.5f;
-            finish(early);
-            if (early) {
-              logT = logT1;
-              if (second) dens = m2 = e.tau = e.cr = e.cg = e.cb = 0.f;
-              else o_dens = o_m2 = 0.f;
-            }
-          }
-          sr = fmaf(e.cr, before, sr);
-          sg = fmaf(e.cg, before, sg);
-          sb = fmaf(e.cb, before, sb);
-          const float dz1 = dz + (second ? o_dens : dens), dw1 = fmaf(second ? o_m2 : m2, 0.5f, dw);
-          dx = fmaf(m2, second ? dz1 : dz, dx);
-          dy = fmaf(dens, second ? dw1 : dw, dy);
-          dv = fmaf(dens, e.tau, dv);
-          dz = dz1 + (second ? dens : o_dens);
-          dw = fmaf(second ? m2 : o_m2, 0.5f, dw1);
         }
       }
       hitbits &= ~(missed | __shfl_xor_sync(FULL, missed, 16));
@@ -973,26 +971,10 @@ __device__ __forceinline__ void walk_unit(
             logT -= e.tau;
             T *= e.alpha;
             finished = logT < -5.5f;
-          } else if (MODE == kConstColor) {
-            const float weight = T * (1.0f - e.alpha);
-            const float mm = tukey_power_ladder(e.enter * pre_multi, ladder_p);
-            dx = fmaf(2.0f * weight * mm, dz, dx);
-            dy = fmaf(weight, dw, dy);
-            dz += weight;
-            dw = fmaf(weight, mm, dw);
-            T *= e.alpha;
-            finished = T < 1.0f / 255.0f;
           } else {
-            logT -= e.tau;
-            T *= e.alpha;
-            const float dens = cb.w;
-            const float m2 = dens * (e.exit + e.enter);  // twice the first moment
-            dx = fmaf(m2, dz, dx);
-            dy = fmaf(dens, dw, dy);
-            dz += dens;
-            dw = fmaf(m2, 0.5f, dw);
-            dv = fmaf(dens, e.tau, dv);
-            finished = logT < -5.5f;
+            const float m2 = MODE == kConstColor ? tukey_power_ladder(e.enter * pre_multi, ladder_p) : cb.w * (e.exit + e.enter);
+            update_state<MODE>(e.tau, e.alpha, cb.w, m2, T, logT, dx, dy, dz, dw, dv);
+            finished = MODE == kConstColor ? T < 1.0f / 255.0f : logT < -5.5f;
           }
           if (finished) {
             active = false;
@@ -1089,14 +1071,6 @@ __device__ __forceinline__ void walk_unit(
   const int64_t pix = (int64_t)u.y * rcam.image_width + u.x;
   if (hit_counts && el == 0 && unit < n_units && RM_INDEX_OK((int64_t)u.tile * u.subs + u.sub, RM_X_UNITS, 4))
     hit_counts[(int64_t)u.tile * u.subs + u.sub] = n_ent;
-  if constexpr (PAIR) {  // T, logT and the running sums dz and dw are the same in both lanes of a pixel
-    sr += __shfl_xor_sync(FULL, sr, 16);
-    sg += __shfl_xor_sync(FULL, sg, 16);
-    sb += __shfl_xor_sync(FULL, sb, 16);
-    dx += __shfl_xor_sync(FULL, dx, 16);
-    dy += __shfl_xor_sync(FULL, dy, 16);
-    dv += __shfl_xor_sync(FULL, dv, 16);
-  }
   dy *= 2.0f;  // the factors common to all terms of these moments
   dv *= 1.0f / 3.0f;
   if (u.inside && !second) {
