@@ -1633,8 +1633,10 @@ k_backward_finish(const int32_t* __restrict__ indices, const float* __restrict__
 // Distortion loss: mean over the pixels of max(0, (d0 - d1 + d4) / max(d2^2, 1e-6)), utils/train_util.py:58-62.
 // One pass over the moments and a fixed-order sum of at most RM_LOSS_PARTIALS block sums, where torch takes nine
 // kernels; bound by HBM for a large frame (20 bytes per pixel), by the two launches for a small one.
+// A NaN passes both clamps, as in torch (fmaxf would drop it): the loss of a frame that has diverged shows it.
 // ----------------------------------------------------------------------------
 constexpr int kLossThreads = 256;
+__device__ __forceinline__ float at_least(float x, float low) { return x < low ? low : x; }
 
 __device__ __forceinline__ float block_sum(float v) {  // valid in thread 0
   __shared__ float s[kLossThreads / 32];
@@ -1657,7 +1659,7 @@ k_distortion_loss(const float* __restrict__ dist, int64_t n, float* __restrict__
   for (int64_t i = (int64_t)blockIdx.x * kLossThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kLossThreads) {
     const float* d = dist + 5 * i;
     const float d2 = __ldg(d + 2);
-    sum += fmaxf(((__ldg(d) - __ldg(d + 1)) + __ldg(d + 4)) / fmaxf(d2 * d2, 1e-6f), 0.0f);
+    sum += at_least(((__ldg(d) - __ldg(d + 1)) + __ldg(d + 4)) / at_least(d2 * d2, 1e-6f), 0.0f);
   }
   const float t = block_sum(sum);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
@@ -1681,11 +1683,12 @@ k_distortion_loss_backward(const float* __restrict__ dist, int64_t n, const floa
   __syncthreads();
   if (threadIdx.x < count) {
     float* d = rows + 5 * threadIdx.x;
-    const float a = (d[0] - d[1]) + d[4], d2 = d[2], sq = d2 * d2, den = fmaxf(sq, 1e-6f), g = __ldg(g_loss) / (float)n;
-    const float g_a = a / den >= 0.0f ? g / den : 0.0f;  // both clamps pass the gradient at their bounds
+    const float a = (d[0] - d[1]) + d[4], d2 = d[2], sq = d2 * d2, den = at_least(sq, 1e-6f), q = a / den;
+    // both clamps pass the gradient at their bounds
+    const float g = q >= 0.0f ? __ldg(g_loss) / (float)n : 0.0f, g_a = g / den;
     d[0] = g_a;
     d[1] = -g_a;
-    d[2] = sq >= 1e-6f ? -2.0f * d2 * g_a * (a / den) : 0.0f;
+    d[2] = 2.0f * d2 * (sq >= 1e-6f ? -g_a * q : 0.0f);
     d[3] = 0.0f;
     d[4] = g_a;
   }
