@@ -30,7 +30,12 @@ class DistortionLoss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):
-        return _lib.native().distortion_loss_backward(ctx.saved_tensors[0], grad_loss)
+        d, = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: a gradient that can be differentiated again, in torch
+            total = (d[:, :, 2] ** 2).clip(min=1e-6)
+            loss = (((d[:, :, 0] - d[:, :, 1]) + d[:, :, 4]) / total).clip(min=0).mean()
+            return torch.autograd.grad(loss, d, grad_loss, create_graph=True)[0]
+        return _lib.native().distortion_loss_backward(d, grad_loss)
 
 
 def render(indices, vertices, cell_values, tcam, ray_jitter=None, before_blend=None):
