@@ -72,14 +72,14 @@ void extents(std::initializer_list<std::pair<int, int64_t>> list) {  // bounds-c
 }
 enum { kList, kTets, kVerts, kHitIds, kHitMasks, kUnits };
 
-// The camera dictionary (data/camera.py:72-91 plus the tile fields of utils/train_util.py:30-37) as an RmCamera, with
-// the device tensors it points at.
+// The camera dictionary (data/camera.py:72-91 plus the tile fields of utils/train_util.py:30-37), or any object with its
+// subscripts and its get, as an RmCamera, with the device tensors it points at.
 struct Camera {
   RmCamera c;
   Tensor keep[4];
   bool band_rows_only;
 
-  Camera(const py::dict& d, const at::Device& device, const py::object& tile_rows) {
+  Camera(const py::object& d, const at::Device& device, const py::object& tile_rows) {
     static const char* names[4] = {"world_view_transform", "K", "cam_pos", "distortion_params"};
     static const int64_t sizes[4] = {16, 9, 3, 4};
     const float** slots[4] = {&c.world_view_transform, &c.K, &c.cam_pos, &c.distortion_params};
@@ -106,13 +106,14 @@ struct Camera {
     c.grid_width = integer("grid_width");
     c.tile_row_begin = 0;
     c.tile_row_end = c.grid_height;
-    py::object rows = !tile_rows.is_none() ? tile_rows : d.contains("tile_rows") ? py::object(d["tile_rows"]) : py::none();
+    const py::object get = d.attr("get");
+    py::object rows = !tile_rows.is_none() ? tile_rows : get("tile_rows", py::none());
     if (!rows.is_none()) {
       c.tile_row_begin = py::int_(py::object(rows[py::int_(0)])).cast<int32_t>();
       c.tile_row_end = py::int_(py::object(rows[py::int_(1)])).cast<int32_t>();
     }
     // a band-restricted call zero-fills the image rows outside its band unless the caller reads the band only
-    band_rows_only = d.contains("band_rows_only") && py::bool_(py::object(d["band_rows_only"])).cast<bool>();
+    band_rows_only = py::bool_(get("band_rows_only", false)).cast<bool>();
   }
 };
 
@@ -290,7 +291,7 @@ Tensor distortion_loss_backward(const Tensor& distortion_img, const Tensor& grad
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<Camera>(m, "Camera")
-      .def(py::init<const py::dict&, const at::Device&, const py::object&>())
+      .def(py::init<const py::object&, const at::Device&, const py::object&>())
       .def_property_readonly("address", [](const Camera& c) { return reinterpret_cast<uintptr_t>(&c.c); })
       .def_property_readonly("band_rows_only", [](const Camera& c) { return c.band_rows_only; })
       .def_property_readonly("grid", [](const Camera& c) { return std::make_tuple(c.c.grid_height, c.c.grid_width); })
