@@ -21,6 +21,9 @@ class AlphaBlendTiledRender(torch.autograd.Function):
         assert tet_density.shape[1] == 7, "cell values are (density, r, g, b, gx, gy, gz) per tet"
         if ray_jitter is not None:  # None: the pixel centres
             assert ray_jitter.shape == (render_grid.image_height, render_grid.image_width, 2)
+            if ray_jitter.dtype != torch.float32 or not ray_jitter.is_contiguous():
+                # once for both directions: the caller may refill a jitter that was copied as soon as this returns
+                ray_jitter = ray_jitter.detach().float().contiguous()
         raster._require_cuda(vertices, "vertices")
         cam = raster.CameraArgs(tcam, vertices.device)
         assert cam.native.grid == (render_grid.grid_height, render_grid.grid_width)
@@ -41,8 +44,6 @@ class AlphaBlendTiledRender(torch.autograd.Function):
     def backward(ctx, grad_output_img, grad_distortion_img, grad_vert_alive):
         (sorted_tetra_idx, tile_ranges, indices, verts, cell, output_img, distortion_img, jitter, n_contributors,
          records, tet_flags, hit_counts, hit_ids, hit_masks) = ctx.saved_tensors
-        if jitter is not None:
-            jitter = jitter.contiguous().float()
         if grad_output_img is None:
             grad_output_img = torch.zeros_like(output_img)
         if grad_distortion_img is None:
