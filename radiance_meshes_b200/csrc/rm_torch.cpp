@@ -148,10 +148,7 @@ std::vector<Tensor> project_and_bin(const Tensor& indices_in, const Tensor& vert
 
 // The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).
 std::tuple<int64_t, int64_t, int64_t, int64_t> wait_info(const Tensor& host_info, const Tensor& vertices) {
-  {
-    py::gil_scoped_release release;
-    c10::cuda::getCurrentCUDAStream(vertices.device().index()).synchronize();
-  }
+  c10::cuda::getCurrentCUDAStream(vertices.device().index()).synchronize();
   const RmBinInfo* r = ptr<RmBinInfo>(host_info);
   return {r->n_keys, r->n_region_keys, r->n_visible, r->status};
 }
@@ -299,13 +296,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         return !(c.c.tile_row_begin == 0 && c.c.tile_row_end == c.c.grid_height) && !c.band_rows_only;
       });
   m.def("bind", &bind);
-  m.def("project_and_bin", &project_and_bin);
-  m.def("wait_info", &wait_info);
-  m.def("build_tile_lists", &build_tile_lists);
-  m.def("pack_records", &pack_records);
-  m.def("forward", &forward);
-  m.def("blend_forward", &blend_forward);
-  m.def("backward", &backward);
-  m.def("distortion_loss", &distortion_loss);
-  m.def("distortion_loss_backward", &distortion_loss_backward);
+  // The interpreter lock is not held while a frame's memory is allocated and its kernels are launched (a launch waits when the
+  // GPU's queue is full): other threads of the program, those of other GPUs among them, go on.
+  py::call_guard<py::gil_scoped_release> unlocked;
+  m.def("project_and_bin", &project_and_bin, unlocked);
+  m.def("wait_info", &wait_info, unlocked);
+  m.def("build_tile_lists", &build_tile_lists, unlocked);
+  m.def("pack_records", &pack_records, unlocked);
+  m.def("forward", &forward, unlocked);
+  m.def("blend_forward", &blend_forward, unlocked);
+  m.def("backward", &backward, unlocked);
+  m.def("distortion_loss", &distortion_loss, unlocked);
+  m.def("distortion_loss_backward", &distortion_loss_backward, unlocked);
 }
