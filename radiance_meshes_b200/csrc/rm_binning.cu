@@ -1047,11 +1047,14 @@ struct BinLayout {
   int64_t nblk_scan_t, nblk_scan_g;
 };
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-// A small tile grid gets several partial difference arrays, one for every so many blocks of the projection: its
+// A small tile grid gets several partial difference arrays, dealt to the blocks of the projection: its
 // atomics otherwise queue on few addresses (614k tets on the 51 x 51 corners of 16 x 16-pixel tiles: k_project
 // 265 us, against 43 us for the same tets on 201 x 201).  128 KB hold 8 copies of that grid and one of any grid
-// larger than 127 x 127, where the queues are short.
-constexpr int64_t kDiffWords = 32768;
+// larger than 127 x 127, where the queues are short; of the smallest grids they hold thousands, which a lane then adds up
+// one after another.  A copy for every two blocks of the projection is enough (projection and rank sort of 13k tets on
+// 2 x 2 corners 330 us with all that fit, 53 with a copy for 256 tets, 66 for 512; 600k tets 488, 222, 177; on 9 x 9
+// corners 46, 39, 37 and 117, 113, 113).
+constexpr int64_t kDiffWords = 32768, kTetsPerDiffCopy = 256;
 BinLayout make_layout(int64_t T, int64_t G, int gh, int gw) {
   BinLayout L;
   size_t off = 0;
@@ -1084,7 +1087,7 @@ BinLayout make_layout(int64_t T, int64_t G, int gh, int gw) {
   // (gh+1)*(gw+1) <= G + gh + gw + 1; gh, gw <= G
   const int64_t n_diff = gh >= 0 ? (int64_t)(gh + 1) * (gw + 1) : 4 * G + 4;
   L.diff_copies = 1;
-  while (2 * L.diff_copies * n_diff <= kDiffWords) L.diff_copies *= 2;
+  while (2 * L.diff_copies * n_diff <= kDiffWords && 2 * L.diff_copies * kTetsPerDiffCopy <= T) L.diff_copies *= 2;
   L.tile_diff = take(4 * (size_t)(n_diff > kDiffWords ? n_diff : kDiffWords));
   L.zero_bytes = L.tile_diff + 4 * (size_t)(L.diff_copies * n_diff) - L.zero;
   L.total = off;
