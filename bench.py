@@ -734,7 +734,7 @@ def run_gpu(args):
                         note="the kernel is bound by instruction issue (ncu: 72 % of the issue slots, DRAM at 3 %), so its HBM "
                              "fraction is low by construction; `fp32_pipe` is its second roofline")
     frame_bytes = sum(alg.values())
-    # Second roofline: the integration kernels are bound by the fp32 pipes, not by HBM.  Pair evaluations x
+    # Second roofline: the integration kernels are bound by instruction issue, not by HBM.  Hits x
     # 170 flop (slab test + segment integral) against 148 SMs x 128 lanes x 2 flop at the sampled SM clock.
     fp32_pipe = None
     if hit_stats and clocks and clocks.get("sm_mhz"):
@@ -743,13 +743,14 @@ def run_gpu(args):
         fp32_pipe = dict(flop_per_pair=170, peak_tflops=peak_tf,
                          forward=dict(pairs_reference_algorithm=hit_stats["walked_pixel_entries"],
                                       pairs_evaluated=hit_stats["pixel_hits"],
-                                      frac=(hit_stats["walked_pixel_entries"] * 170 / (fwd_ms * 1e-3) / 1e12 / peak_tf)
+                                      frac=(hit_stats["pixel_hits"] * 170 / (fwd_ms * 1e-3) / 1e12 / peak_tf)
                                       if fwd_ms else None),
                          backward=dict(pairs=hit_stats["pixel_hits"],
                                        frac=(hit_stats["pixel_hits"] * 2 * 170 / (bwd_ms * 1e-3) / 1e12 / peak_tf)
                                        if bwd_ms else None),
-                         note="forward: the reference algorithm's pair evaluations (sum of n_contributors) per second of "
-                              "k_forward; backward: hits x (re-evaluation + reverse, counted as 2 x 170 flop)")
+                         note="forward: (pixel, tet) hits x 170 flop per second of k_forward (the reference algorithm evaluates "
+                              "all of pairs_reference_algorithm, the sum of n_contributors); backward: hits x (re-evaluation + "
+                              "reverse, counted as 2 x 170 flop)")
     line = dict(
         metric="fwd+bwd Mpix/s at 1080p, 6.5M tets", value=value, unit="Mpix/s", n_gpus=world, steps=args.steps,
         warmup=args.warmup, ms_per_step=ms_step, higher_is_better=True, scaling="weak", vs_baseline=None,

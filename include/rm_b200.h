@@ -35,8 +35,9 @@ extern "C" {
 #define RM_STATUS_BAD_INDEX 4u    /* a tet names a vertex outside [0, n_vertices): the tet is treated as culled
                                      (the reference would read out of bounds) */
 
-/* Floats per packed tet record (24 used by the integration + 12 for the hull edge
- * lines of the projected tet, used to cull whole tiles) and per record-gradient row. */
+/* Floats to allocate per packed tet record, and per record-gradient row.  A record is 24 floats for the integration and 8
+ * for the hull lines of the projected tet; records 2k and 2k + 1 lie one behind the other in the 72 floats of the pair, so
+ * that each starts on a 32-byte sector: record t at float 36 t - 4 (t & 1). */
 #define RM_RECORD_FLOATS 36
 #define RM_GRAD_RECORD_FLOATS 24
 

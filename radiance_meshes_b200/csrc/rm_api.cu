@@ -15,8 +15,7 @@ size_t rm_bin_layout_bytes(int64_t, int64_t);
 int rm_launch_bin_prepare(int64_t, const RmCamera*, void*, size_t, uint32_t**, int32_t**, int*, uint32_t**, uint32_t**,
                           cudaStream_t);
 int rm_launch_bin_finish(int64_t, const RmCamera*, const int32_t*, int32_t*, RmBinInfo*, RmBinInfo*, void*, cudaStream_t);
-int rm_launch_build_lists(const int32_t*, const int32_t*, int64_t, const RmCamera*, int64_t, int64_t, void*, void*, size_t,
-                          int32_t*, cudaStream_t);
+int rm_launch_build_lists(int64_t, const RmCamera*, int64_t, int64_t, void*, void*, size_t, int32_t*, cudaStream_t);
 size_t rm_list_plan_bytes(int64_t, int, int);
 int rm_launch_pack(const int32_t*, const float*, const float*, int64_t, int64_t, const RmCamera*, const int32_t*,
                    float*, uint8_t*, uint8_t*, cudaStream_t);
@@ -239,8 +238,9 @@ int rm_build_tile_lists(const int32_t* rect_tile_space, const int32_t* tile_rang
   if (!rm_aligned16(rect_tile_space)) return RM_ERR_WORKSPACE;
   rc = rm_bind_device(workspace);
   if (rc) return rc;
-  return rm_launch_build_lists(rect_tile_space, tile_ranges, n_tets, cam, n_keys, n_region_keys, workspace, scratch,
-                               scratch_bytes, sorted_tetra_idx, static_cast<cudaStream_t>(stream));
+  // (the first half has left the rectangles, in rank order, and the tiles' starts in the workspace)
+  return rm_launch_build_lists(n_tets, cam, n_keys, n_region_keys, workspace, scratch, scratch_bytes, sorted_tetra_idx,
+                               static_cast<cudaStream_t>(stream));
 }
 
 int rm_pack_records(const int32_t* indices, const float* vertices, const float* cell_values, int64_t n_tets,

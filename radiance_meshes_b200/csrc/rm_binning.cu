@@ -1222,6 +1222,8 @@ bool make_list_plan(int64_t n_region_keys, int gh, int gw, ListPlan* P) {
 }
 }  // namespace
 
+// A kernel for every width of digit: with 8-bit digits throughout, whatever the number of regions, the passes took 222 us in
+// place of 197 (6M tets, 4,080 regions: two of 6 bits) and 1079 in place of 1012 (36M, 16,200 regions: two of 7).
 template <int ITEMS>
 static auto pass_kernel(int bits) {
   static decltype(&rm::k_region_pass<1, ITEMS>) const kernels[rm::kRadixBits + 1] = {
@@ -1237,11 +1239,8 @@ size_t rm_list_plan_bytes(int64_t n_region_keys, int gh, int gw) {
   return P.total;
 }
 
-int rm_launch_build_lists(const int32_t* rect, const int32_t* tile_ranges, int64_t T, const RmCamera* cam,
-                          int64_t n_keys, int64_t n_region_keys, void* ws, void* scratch, size_t scratch_bytes,
-                          int32_t* sorted_idx, cudaStream_t st) {
-  (void)tile_ranges;
-  (void)rect;  // the rectangles were put in rank order by the first half
+int rm_launch_build_lists(int64_t T, const RmCamera* cam, int64_t n_keys, int64_t n_region_keys, void* ws, void* scratch,
+                          size_t scratch_bytes, int32_t* sorted_idx, cudaStream_t st) {
   if (n_keys == 0) return RM_OK;
   const int gh = cam->grid_height, gw = cam->grid_width;
   const int64_t G = (int64_t)gh * gw;

@@ -17,16 +17,16 @@
 //     The per-pixel origin offset o = cam + min_t*d only shifts each plane
 //     distance by min_t*(n_i.d), so the per-(pixel,tet) work drops from four
 //     cross products to four dot products.
-//   * A half-warp owns 16 pixels of one tile; a warp therefore walks two tile
-//     lists side by side.  Forward: the list is examined 16 entries at a time
-//     (hull lines against the box of the half-warp's samples); survivors are
+//   * 16 pixels of one tile are a unit, walked by a half-warp or, two lanes per
+//     pixel, by a warp.  Forward: the list is examined one entry per lane
+//     (hull lines against the box of the unit's samples); survivors are
 //     tested against each of the 16 sample positions, which gives the mask of
-//     pixels a tet can cover; entries with a non-empty mask are staged 16 at a
-//     time with 128-bit cp.async copies, double buffered, and every lane then
-//     walks only the staged entries that cover its pixel.  A half-warp stops as
-//     soon as all of its pixels have terminated.  Every evaluated batch is
+//     pixels a tet can cover; entries with a non-empty mask are staged in batches
+//     with 128-bit cp.async copies that land while the next ones are examined, and
+//     every lane then walks only the staged entries that cover its pixel.  A unit
+//     stops as soon as all of its pixels have terminated.  Every evaluated batch is
 //     appended, with the per-pixel bit sets of the entries that were hit, to the
-//     half-warp's hit list.
+//     unit's hit list.
 //   * Backward walks the hit lists back to front: a lane per pixel evaluates the hits
 //     and reduces each to seven scalars, then a lane per entry sums them over the 16
 //     pixels into a per-tet row of record gradients; a per-tet kernel applies the chain
