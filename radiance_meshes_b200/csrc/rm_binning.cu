@@ -212,8 +212,9 @@ __device__ __noinline__ void run_tile_job(const TileJob& j) {
 // blocks before it (decoupled look-back: Merrill and Garland, "Single-pass parallel prefix scan with decoupled
 // look-back", 2016).  Blocks number themselves with a ticket, so those a block waits for are running already.  The
 // first pass drops the culled tets (key 0xFFFFFFFF), the others run over the visible ones.
-// Bound by HBM: 16 bytes per tet and pass.  Histogram, row scan and scatter launches for each pass, over all tets: 248 us
-// for 6M tets, 1.2 ms for 30M; this 150 us and 0.70 ms.
+// 16 bytes per tet and pass; bound by the issue of the ballot ranking and the latency of a block's phases (issue slots 41 %,
+// alu pipe 48 %, DRAM 7 %).  Histogram, row scan and scatter launches for each pass, over all tets: 248 us for 6.7M tets,
+// 1.2 ms for 36M; this, with the tile populations on the way, 224 us and 0.88 ms.
 // ---------------------------------------------------------------------------
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
@@ -310,9 +311,9 @@ __device__ __forceinline__ uint32_t finish_look_back(uint32_t before, const uint
 
 // Sum of what the `blocks` blocks before `word` hold, the nearest first, `stride` words apart.  AHEAD words are asked for
 // at a time: blocks that run together all walk over each other's runs, one round trip to L2 per word otherwise.  Two are
-// best for the rank sort (30M tets: 1016, 934, 1041 us with 1, 2, 8), whose blocks hold many words each, eight for the
-// list build (passes 592 -> 520 us each, lists 1683 -> 1551 us).  finish(before, word, blocks), where a wait runs out, is a
-// call that ends the walk: with the counting inside the loop the rank sort of 30M tets took 1065 us in place of 897.
+// enough for the rank sort (36M tets: 975, 881, 881 us with 1, 2, 8), whose blocks hold many words each, eight are better
+// for the list build (two passes 1180 -> 1012 us, lists 1681 -> 1554 us).  finish(before, word, blocks), where a wait runs
+// out, is a call that ends the walk: with the counting inside the loop the rank sort of 36M tets took 1065 us, not 881.
 template <uint32_t AHEAD, typename F>
 __device__ __forceinline__ uint32_t look_back(const uint32_t* word, uint32_t blocks, int stride, F finish) {
   uint32_t before = 0;
@@ -940,7 +941,7 @@ __device__ __forceinline__ uint32_t region_of_chunk(const uint32_t* chunk_base, 
 // (look-back, as in the sort passes, blocks numbered by a ticket); and writes tile after tile, 32 consecutive list entries
 // per store.  Bound by the issue of shared-memory and store instructions.  The lists were written straight from the
 // entries before, one store of the covering lanes per round and tile, after a counting launch and one for the cursors:
-// 462 us for the three at 6M tets, 1080p (142M list entries), 2.85 ms at 30M, 2160p (886M); this 275 us and 1.55 ms.
+// 462 us for the three at 6.7M tets, 1080p (142M list entries), 2.85 ms at 36M, 2160p (886M); this 281 us and 1.55 ms.
 constexpr int kFineRounds = kChunk / 32;
 constexpr int kFineStride = kChunk + 4;  // bytes per tile: the lanes' byte stores fall into different banks
 
