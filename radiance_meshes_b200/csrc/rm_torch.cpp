@@ -117,11 +117,31 @@ struct Camera {
   }
 };
 
-// Stage 1 and tile populations.  Returns (indices, vertices, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges,
-// info, workspace, visible[, host_info]).  host_info, if asked for, is page-locked and holds a copy of info once the stream
-// is there: the caller waits for that (wait_info) before it lets go of it.
-std::vector<Tensor> project_and_bin(const Tensor& indices_in, const Tensor& vertices_in, uintptr_t cam_address,
-                                    bool want_host_info) {
+// A copy of a frame's info block in page-locked memory, which the device writes once the stream is there.  The memory goes
+// back only after that, also where a frame is given up in between: it would otherwise be somebody else's by then.
+struct PendingInfo {
+  Tensor block;
+  c10::cuda::CUDAStream stream;
+  bool arrived = false;
+
+  explicit PendingInfo(c10::cuda::CUDAStream s)
+      : block(at::empty({3}, at::TensorOptions().dtype(at::kLong).pinned_memory(true))), stream(s) {}
+  ~PendingInfo() {
+    if (!arrived) cudaStreamSynchronize(stream.stream());
+  }
+  // The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).
+  std::tuple<int64_t, int64_t, int64_t, int64_t> wait() {
+    if (!arrived) stream.synchronize();
+    arrived = true;
+    const RmBinInfo* r = ptr<RmBinInfo>(block);
+    return {r->n_keys, r->n_region_keys, r->n_visible, r->status};
+  }
+};
+
+// Stage 1 and tile populations.  Returns ((indices, vertices, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges,
+// info, workspace, visible), host copy of info if asked for).
+std::tuple<std::vector<Tensor>, std::unique_ptr<PendingInfo>> project_and_bin(const Tensor& indices_in, const Tensor& vertices_in,
+                                                                              uintptr_t cam_address, bool want_host_info) {
   require_cuda(indices_in, "indices");
   require_cuda(vertices_in, "vertices");
   const RmCamera* cam = camera(cam_address);
@@ -134,23 +154,16 @@ std::vector<Tensor> project_and_bin(const Tensor& indices_in, const Tensor& vert
   Tensor tile_ranges = empty({G, 2}, at::kInt, dev), visible = empty({T}, at::kBool, dev);
   const int64_t bytes = (int64_t)lib.rm_bin_workspace_bytes(T, G);
   Tensor info = empty({3}, at::kLong, dev), workspace = empty({bytes}, at::kByte, dev);
-  c10::optional<Tensor> host_info;
-  if (want_host_info) host_info = at::empty({3}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  std::unique_ptr<PendingInfo> pending;
+  if (want_host_info) pending = std::make_unique<PendingInfo>(c10::cuda::getCurrentCUDAStream(dev.index()));
   check(lib.rm_project_and_bin_visible(ptr<int32_t>(indices), T, ptr<float>(vertices), V, cam, ptr<int32_t>(tiles_touched),
                                        ptr<int32_t>(rect), ptr<float>(vs_tetra), ptr<float>(circumcenter),
                                        ptr<int32_t>(tile_ranges), ptr<RmBinInfo>(info), workspace.data_ptr(), bytes,
-                                       ptr<uint8_t>(visible), ptr<RmBinInfo>(host_info), stream_of(vertices)));
+                                       ptr<uint8_t>(visible), pending ? ptr<RmBinInfo>(pending->block) : nullptr,
+                                       stream_of(vertices)));
   std::vector<Tensor> out = {indices, vertices, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges, info, workspace,
                              visible};
-  if (want_host_info) out.push_back(*host_info);
-  return out;
-}
-
-// The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).
-std::tuple<int64_t, int64_t, int64_t, int64_t> wait_info(const Tensor& host_info, const Tensor& vertices) {
-  c10::cuda::getCurrentCUDAStream(vertices.device().index()).synchronize();
-  const RmBinInfo* r = ptr<RmBinInfo>(host_info);
-  return {r->n_keys, r->n_region_keys, r->n_visible, r->status};
+  return {std::move(out), std::move(pending)};
 }
 
 Tensor build_tile_lists(const Tensor& rect, const Tensor& tile_ranges, const Tensor& workspace, uintptr_t cam_address,
@@ -299,8 +312,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // The interpreter lock is not held while a frame's memory is allocated and its kernels are launched (a launch waits when the
   // GPU's queue is full): other threads of the program, those of other GPUs among them, go on.
   py::call_guard<py::gil_scoped_release> unlocked;
+  py::class_<PendingInfo>(m, "PendingInfo").def("wait", &PendingInfo::wait, unlocked);
   m.def("project_and_bin", &project_and_bin, unlocked);
-  m.def("wait_info", &wait_info, unlocked);
   m.def("build_tile_lists", &build_tile_lists, unlocked);
   m.def("pack_records", &pack_records, unlocked);
   m.def("forward", &forward, unlocked);

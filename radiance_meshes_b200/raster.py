@@ -46,22 +46,22 @@ def _require_cuda(t, name):
 
 def project_and_bin(indices, vertices, tcam, tile_rows=None, host_info=False):
     """Stage 1 and tile populations. Returns a dict of outputs plus the binning context.  With `host_info` the counters
-    also arrive in page-locked memory: the caller must call read_info(ctx) before it drops the context."""
+    also arrive in page-locked memory, where read_info(ctx) finds them without a copy."""
     _require_cuda(indices, "indices")
     _require_cuda(vertices, "vertices")
     cam = CameraArgs(tcam, vertices.device, tile_rows)
-    out = _lib.native().project_and_bin(indices, vertices, cam.address, host_info)
-    indices, verts, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges, info, ws, visible = out[:10]
+    out, pending = _lib.native().project_and_bin(indices, vertices, cam.address, host_info)
+    indices, verts, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges, info, ws, visible = out
     gh, gw = cam.native.grid
     return dict(indices=indices, vertices=verts, cam=cam, tiles_touched=tiles_touched, rect=rect, vs_tetra=vs_tetra,
                 circumcenter=circumcenter, tile_ranges=tile_ranges, info=info, workspace=ws, visible=visible,
-                host_info=out[10] if host_info else None, T=indices.shape[0], V=verts.shape[0], G=gh * gw)
+                host_info=pending, T=indices.shape[0], V=verts.shape[0], G=gh * gw)
 
 
 def read_info(ctx):
     """The one host synchronisation of the binning stage: N, visible count, status."""
     if ctx.get("host_info") is not None:
-        n_keys, ctx["n_region_keys"], n_visible, status = _lib.native().wait_info(ctx["host_info"], ctx["vertices"])
+        n_keys, ctx["n_region_keys"], n_visible, status = ctx["host_info"].wait()
     else:
         n_keys, ctx["n_region_keys"], second = ctx["info"].tolist()
         n_visible = second & 0xFFFFFFFF
