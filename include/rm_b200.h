@@ -74,7 +74,8 @@ typedef struct RmBinInfo {
  * Hit lists, written by rm_forward and walked by rm_backward (device pointers).  No
  * counterpart in the reference, whose backward pass walks every tile list again and
  * repeats every intersection test.  A unit is one group of 16 pixels of a tile (tile t,
- * group s of S = ceil(tile_width*tile_height / 16): unit t*S + s).  The forward pass
+ * group s of S = ceil(tile_width*tile_height / 16): unit t*S + s; where both sides of a
+ * tile are multiples of 4 a group is a block of 4 x 4).  The forward pass
  * evaluates a unit's list in batches of 16 entries that can cover one of its pixels (the
  * last batch may hold fewer) and records every batch, in list order:
  *   counts[G*S] i32        number of recorded entries of the unit

@@ -493,6 +493,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 constexpr int kWarpsPerBlock = 4;
 
+// 16 pixels of a tile: a block of 4 x 4 where tiles divide into such blocks, else 16 in the order of the tile's rows.  A block
+// is touched by fewer tets than a strip, and more of its pixels by each (600k tets, 800 x 800, constant colour, 16 x 16
+// tiles: 658 -> 549 us with blocks in place of strips of 16 x 1).
 struct Unit {
   int tile;       // linear tile index
   int x, y;       // pixel
@@ -517,8 +520,16 @@ __device__ __forceinline__ Unit make_unit(const RmCamera& c, const int2* __restr
   u.tile = c.tile_row_begin * c.grid_width + (int)t;
   int ty = u.tile / c.grid_width, tx = u.tile - ty * c.grid_width;
   u.sub = sub;
-  int p = sub * 16 + lane16;
-  int ly = p / c.tile_width, lx = p - ly * c.tile_width;
+  int lx, ly;
+  if (((c.tile_width | c.tile_height) & 3) == 0) {
+    const int across = c.tile_width >> 2, by = sub / across;
+    lx = 4 * (sub - by * across) + (lane16 & 3);
+    ly = 4 * by + (lane16 >> 2);
+  } else {
+    const int p = sub * 16 + lane16;
+    ly = p / c.tile_width;
+    lx = p - ly * c.tile_width;
+  }
   u.x = tx * c.tile_width + lx;
   u.y = ty * c.tile_height + ly;
   u.inside = ly < c.tile_height && u.x < c.image_width && u.y < c.image_height;
