@@ -116,132 +116,188 @@ __device__ __forceinline__ void make_planes(const f3 v[4], f3 cam, PlaneSetup& p
 
 constexpr int kPackThreads = 128;
 
-// One thread per tet builds the record in registers; the block then writes its
-// records through shared memory so that the global stores are contiguous.
+// Record of tet g, whose vertices are `id`.
+__device__ __forceinline__ void build_record(float4* r, int4 id, const float* __restrict__ vertices, const float* __restrict__ cell,
+                                             int64_t g, float density, const RmCamera& rcam) {
+  f3 cam = {__ldg(rcam.cam_pos), __ldg(rcam.cam_pos + 1), __ldg(rcam.cam_pos + 2)};
+  f3 v[4] = {load3(vertices, id.x), load3(vertices, id.y), load3(vertices, id.z), load3(vertices, id.w)};
+  PlaneSetup p;
+  make_planes(v, cam, p);
+  const float* c = cell + 7 * g;
+  f3 base = {__ldg(c + 1), __ldg(c + 2), __ldg(c + 3)};
+  f3 grd = {__ldg(c + 4), __ldg(c + 5), __ldg(c + 6)};
+  float s0 = dot_fma(grd, cam - v[0]);
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {  // planes in pairs: operands of the packed arithmetic of the slab test
+    r[i] = make_float4(p.n[i].x, p.n[i + 1].x, p.n[i].y, p.n[i + 1].y);
+    r[i + 1] = make_float4(p.n[i].z, p.n[i + 1].z, -p.D[i], -p.D[i + 1]);
+  }
+  r[4] = make_float4(grd.x, grd.y, grd.z, s0);
+  r[5] = make_float4(base.x, base.y, base.z, density);
+  // Vertices in pixel coordinates.  Only meaningful with the whole tet in front of the camera; otherwise the cull is
+  // disabled for this tet (NaN lines).
+  const float* W = rcam.world_view_transform;
+  const float fx = __ldg(rcam.K + 0), cx = __ldg(rcam.K + 2), fy = __ldg(rcam.K + 4), cy = __ldg(rcam.K + 5);
+  float px[4], py[4];
+  bool ok = true;
+  // Bound of the fp32 rounding error of the projected vertices, in pixels: the camera-space
+  // coordinates are sums of four products (error <= 4 * 2^-24 * sum of magnitudes), and the error of
+  // X/Z grows with 1/Z, so vertices near the camera plane project with errors far above the 0.01
+  // pixel margin of the hull tests.  The lines are moved outwards by the bound (two end points per
+  // line); a tet whose bound reaches half a pixel, or with a vertex behind the near plane, is not culled.
+  float perr = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float X = __ldg(W + 0) * v[k].x + __ldg(W + 1) * v[k].y + __ldg(W + 2) * v[k].z + __ldg(W + 3);
+    float Y = __ldg(W + 4) * v[k].x + __ldg(W + 5) * v[k].y + __ldg(W + 6) * v[k].z + __ldg(W + 7);
+    float Z = __ldg(W + 8) * v[k].x + __ldg(W + 9) * v[k].y + __ldg(W + 10) * v[k].z + __ldg(W + 11);
+    const float u4 = 2.4e-7f;
+    const float eX = u4 * (fabsf(__ldg(W + 0) * v[k].x) + fabsf(__ldg(W + 1) * v[k].y) + fabsf(__ldg(W + 2) * v[k].z) + fabsf(__ldg(W + 3)));
+    const float eY = u4 * (fabsf(__ldg(W + 4) * v[k].x) + fabsf(__ldg(W + 5) * v[k].y) + fabsf(__ldg(W + 6) * v[k].z) + fabsf(__ldg(W + 7)));
+    const float eZ = u4 * (fabsf(__ldg(W + 8) * v[k].x) + fabsf(__ldg(W + 9) * v[k].y) + fabsf(__ldg(W + 10) * v[k].z) + fabsf(__ldg(W + 11)));
+    ok = ok && Z > 1e-3f;
+    const float iz = 1.0f / Z;
+    px[k] = fx * (X * iz) + cx;
+    py[k] = fy * (Y * iz) + cy;
+    const float ex = fabsf(fx) * iz * (eX + fabsf(X * iz) * eZ) + 4e-7f * (fabsf(px[k]) + fabsf(cx));
+    const float ey = fabsf(fy) * iz * (eY + fabsf(Y * iz) * eZ) + 4e-7f * (fabsf(py[k]) + fabsf(cy));
+    perr = fmaxf(perr, ex + ey);
+  }
+  const float margin = 2.0f * perr;
+  ok = ok && margin < 0.5f;
+  // A vertex pair is a hull edge iff the other two vertices lie on one side of its line; a tet projects to a
+  // quadrilateral (4 such pairs) or to a triangle with one vertex inside (3).  Anything else is degenerate and
+  // disables the cull for this tet.
+  float lab[4] = {0, 0, 0, 0}, lc[4] = {0, 0, 0, 0};
+  int ne = 0;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+#pragma unroll
+    for (int b = a + 1; b < 4; ++b) {
+      const int c1 = (a != 0 && b != 0) ? 0 : ((a != 1 && b != 1) ? 1 : 2);
+      const int c2 = 6 - a - b - c1;
+      const float nx = -(py[b] - py[a]), ny = px[b] - px[a];
+      const float len2 = nx * nx + ny * ny;
+      const float s1 = nx * (px[c1] - px[a]) + ny * (py[c1] - py[a]);
+      const float s2 = nx * (px[c2] - px[a]) + ny * (py[c2] - py[a]);
+      const bool pos = s1 >= 0.0f && s2 >= 0.0f && (s1 > 0.0f || s2 > 0.0f);
+      const bool neg = s1 <= 0.0f && s2 <= 0.0f && (s1 < 0.0f || s2 < 0.0f);
+      if ((pos || neg) && len2 > 0.0f) {
+        const float inv = pos ? rsqrtf(len2) : -rsqrtf(len2);
+        const float ab = pack_normal(nx * inv, ny * inv);
+        const float2 n = unpack_normal(ab);
+        const float low = fminf(fminf(n.x * px[0] + n.y * py[0], n.x * px[1] + n.y * py[1]),
+                                fminf(n.x * px[2] + n.y * py[2], n.x * px[3] + n.y * py[3]));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // slot `ne`, without dynamic indexing
+          if (q == ne) { lab[q] = ab; lc[q] = fmaf(margin, kLineUnit, -low); }
+        }
+        ++ne;
+      }
+    }
+  }
+  ok = ok && (ne == 3 || ne == 4);
+  if (ne == 3) { lab[3] = lab[2]; lc[3] = lc[2]; }
+  if (!ok) {
+    const float qnan = __int_as_float(0x7fc00000);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) lc[k] = qnan;
+  }
+  r[6] = make_float4(lab[0], lc[0], lab[1], lc[1]);
+  r[7] = make_float4(lab[2], lc[2], lab[3], lc[3]);
+}
+
+// A thread builds one record in registers; the block then writes its records through shared memory, so that the global stores
+// are contiguous.  What of a record is written: nothing for a culled tet, which appears in no list; the lines' sector for a
+// tet of zero density (a mark), which the integration kernels drop by its first line without reading more (40 % of the tets of
+// an unbounded scene); else all of it.
+// PER = 1: a thread per tet.  PER > 1: the block first looks at PER tets per thread and makes lists of those to be written
+// whole and of those to be marked, so that all lanes of a warp have a record to build (of 6M tets 46 % have one: 19 lanes of 32
+// had something to do, now 25).
+template <int PER>
 __global__ void __launch_bounds__(kPackThreads, 8)
 k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ vertices,
                const float* __restrict__ cell, int64_t T, int64_t V, RmCamera rcam,
                const int32_t* __restrict__ tiles_touched, float4* __restrict__ records, uint8_t* __restrict__ clear_a,
                uint8_t* __restrict__ clear_b) {
   constexpr int kRow = 9;  // 8 used; the odd stride spreads the rows over the banks
+  constexpr int kTets = PER * kPackThreads;
   __shared__ __align__(16) float4 sm[kPackThreads * kRow];
-  // what of a record is written: nothing for a culled tet, which appears in no list; the lines' sector for a tet of zero
-  // density, which the integration kernels drop by its first line without reading more (40 % of the tets of an unbounded
-  // scene); else all of it
-  enum { kNone, kMark, kAll };
-  __shared__ uint8_t packed[kPackThreads];
-  const int64_t g0 = (int64_t)blockIdx.x * kPackThreads;
-  const int64_t g = g0 + threadIdx.x;
+  __shared__ uint16_t whole[kTets], marks[kTets];
+  __shared__ int n_whole, n_marks;
+  const int64_t g0 = (int64_t)blockIdx.x * kTets;
+  const int lane = threadIdx.x & 31;
   float4* r = sm + threadIdx.x * kRow;
-  const bool live = g < T && !(tiles_touched && tiles_touched[g] == 0);
-  const float density = live ? fmaxf(__ldg(cell + 7 * g), 0.0f) : 0.0f;
-  if (g < T && clear_a) clear_a[g] = 0;
-  if (g < T && clear_b) clear_b[g] = 0;
-  int4 id = make_int4(0, 0, 0, 0);
-  bool ids_ok = false;
-  if (density > 0.0f) {
-    id = __ldg(reinterpret_cast<const int4*>(indices) + g);
-    // a tet that names a vertex outside the table (the projection stage culls it and reports it) is marked like one of
-    // zero density: no pixel can hit it
-    ids_ok = (uint32_t)id.x < (uint64_t)V && (uint32_t)id.y < (uint64_t)V && (uint32_t)id.z < (uint64_t)V &&
-             (uint32_t)id.w < (uint64_t)V;
+  if (PER > 1 && threadIdx.x == 0) n_whole = n_marks = 0;
+  bool live[PER], ids_ok[PER];
+  float density[PER];
+  int4 id[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int64_t g = g0 + k * kPackThreads + threadIdx.x;
+    live[k] = g < T && !(tiles_touched && tiles_touched[g] == 0);
+    if (g < T && clear_a) clear_a[g] = 0;
+    if (g < T && clear_b) clear_b[g] = 0;
   }
-  packed[threadIdx.x] = !live ? kNone : ids_ok ? kAll : kMark;
-  r[6] = make_float4(0.0f, never_seen(), 0.0f, 0.0f);
-  r[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (ids_ok) {
-    f3 cam = {__ldg(rcam.cam_pos), __ldg(rcam.cam_pos + 1), __ldg(rcam.cam_pos + 2)};
-    f3 v[4] = {load3(vertices, id.x), load3(vertices, id.y), load3(vertices, id.z), load3(vertices, id.w)};
-    PlaneSetup p;
-    make_planes(v, cam, p);
-    const float* c = cell + 7 * g;
-    f3 base = {__ldg(c + 1), __ldg(c + 2), __ldg(c + 3)};
-    f3 grd = {__ldg(c + 4), __ldg(c + 5), __ldg(c + 6)};
-    float s0 = dot_fma(grd, cam - v[0]);
 #pragma unroll
-    for (int i = 0; i < 4; i += 2) {  // planes in pairs: operands of the packed arithmetic of the slab test
-      r[i] = make_float4(p.n[i].x, p.n[i + 1].x, p.n[i].y, p.n[i + 1].y);
-      r[i + 1] = make_float4(p.n[i].z, p.n[i + 1].z, -p.D[i], -p.D[i + 1]);
+  for (int k = 0; k < PER; ++k)
+    density[k] = live[k] ? fmaxf(__ldg(cell + 7 * (g0 + k * kPackThreads + threadIdx.x)), 0.0f) : 0.0f;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    ids_ok[k] = false;
+    if (density[k] > 0.0f) {
+      // a tet that names a vertex outside the table (the projection stage culls it and reports it) is marked like one of
+      // zero density: no pixel can hit it
+      id[k] = __ldg(reinterpret_cast<const int4*>(indices) + g0 + k * kPackThreads + threadIdx.x);
+      ids_ok[k] = (uint32_t)id[k].x < (uint64_t)V && (uint32_t)id[k].y < (uint64_t)V && (uint32_t)id[k].z < (uint64_t)V &&
+                  (uint32_t)id[k].w < (uint64_t)V;
     }
-    r[4] = make_float4(grd.x, grd.y, grd.z, s0);
-    r[5] = make_float4(base.x, base.y, base.z, density);
-    // Vertices in pixel coordinates.  Only meaningful with the whole tet in front of the camera; otherwise the cull is
-    // disabled for this tet (NaN lines).
-    const float* W = rcam.world_view_transform;
-    const float fx = __ldg(rcam.K + 0), cx = __ldg(rcam.K + 2), fy = __ldg(rcam.K + 4), cy = __ldg(rcam.K + 5);
-    float px[4], py[4];
-    bool ok = true;
-    // Bound of the fp32 rounding error of the projected vertices, in pixels: the camera-space
-    // coordinates are sums of four products (error <= 4 * 2^-24 * sum of magnitudes), and the error of
-    // X/Z grows with 1/Z, so vertices near the camera plane project with errors far above the 0.01
-    // pixel margin of the hull tests.  The lines are moved outwards by the bound (two end points per
-    // line); a tet whose bound reaches half a pixel, or with a vertex behind the near plane, is not culled.
-    float perr = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float X = __ldg(W + 0) * v[k].x + __ldg(W + 1) * v[k].y + __ldg(W + 2) * v[k].z + __ldg(W + 3);
-      float Y = __ldg(W + 4) * v[k].x + __ldg(W + 5) * v[k].y + __ldg(W + 6) * v[k].z + __ldg(W + 7);
-      float Z = __ldg(W + 8) * v[k].x + __ldg(W + 9) * v[k].y + __ldg(W + 10) * v[k].z + __ldg(W + 11);
-      const float u4 = 2.4e-7f;
-      const float eX = u4 * (fabsf(__ldg(W + 0) * v[k].x) + fabsf(__ldg(W + 1) * v[k].y) + fabsf(__ldg(W + 2) * v[k].z) + fabsf(__ldg(W + 3)));
-      const float eY = u4 * (fabsf(__ldg(W + 4) * v[k].x) + fabsf(__ldg(W + 5) * v[k].y) + fabsf(__ldg(W + 6) * v[k].z) + fabsf(__ldg(W + 7)));
-      const float eZ = u4 * (fabsf(__ldg(W + 8) * v[k].x) + fabsf(__ldg(W + 9) * v[k].y) + fabsf(__ldg(W + 10) * v[k].z) + fabsf(__ldg(W + 11)));
-      ok = ok && Z > 1e-3f;
-      const float iz = 1.0f / Z;
-      px[k] = fx * (X * iz) + cx;
-      py[k] = fy * (Y * iz) + cy;
-      const float ex = fabsf(fx) * iz * (eX + fabsf(X * iz) * eZ) + 4e-7f * (fabsf(px[k]) + fabsf(cx));
-      const float ey = fabsf(fy) * iz * (eY + fabsf(Y * iz) * eZ) + 4e-7f * (fabsf(py[k]) + fabsf(cy));
-      perr = fmaxf(perr, ex + ey);
+  }
+  if constexpr (PER == 1) {
+    enum { kNone, kMark, kAll };
+    const int64_t g = g0 + threadIdx.x;
+    whole[threadIdx.x] = !live[0] ? kNone : ids_ok[0] ? kAll : kMark;
+    r[6] = make_float4(0.0f, never_seen(), 0.0f, 0.0f);
+    r[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (ids_ok[0]) build_record(r, id[0], vertices, cell, g, density[0], rcam);
+    __syncthreads();
+    const int n_rec = (int)min((int64_t)kPackThreads, T - g0);
+    for (int i = threadIdx.x; i < n_rec * 8; i += kPackThreads) {
+      const int row = i >> 3, k = i & 7;
+      if (whole[row] == kAll || (whole[row] == kMark && k >= kLinesAt)) records[record_at(g0 + row) + k] = sm[row * kRow + k];
     }
-    const float margin = 2.0f * perr;
-    ok = ok && margin < 0.5f;
-    // A vertex pair is a hull edge iff the other two vertices lie on one side of its line; a tet projects to a
-    // quadrilateral (4 such pairs) or to a triangle with one vertex inside (3).  Anything else is degenerate and
-    // disables the cull for this tet.
-    float lab[4] = {0, 0, 0, 0}, lc[4] = {0, 0, 0, 0};
-    int ne = 0;
+  } else {
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-#pragma unroll
-      for (int b = a + 1; b < 4; ++b) {
-        const int c1 = (a != 0 && b != 0) ? 0 : ((a != 1 && b != 1) ? 1 : 2);
-        const int c2 = 6 - a - b - c1;
-        const float nx = -(py[b] - py[a]), ny = px[b] - px[a];
-        const float len2 = nx * nx + ny * ny;
-        const float s1 = nx * (px[c1] - px[a]) + ny * (py[c1] - py[a]);
-        const float s2 = nx * (px[c2] - px[a]) + ny * (py[c2] - py[a]);
-        const bool pos = s1 >= 0.0f && s2 >= 0.0f && (s1 > 0.0f || s2 > 0.0f);
-        const bool neg = s1 <= 0.0f && s2 <= 0.0f && (s1 < 0.0f || s2 < 0.0f);
-        if ((pos || neg) && len2 > 0.0f) {
-          const float inv = pos ? rsqrtf(len2) : -rsqrtf(len2);
-          const float ab = pack_normal(nx * inv, ny * inv);
-          const float2 n = unpack_normal(ab);
-          const float low = fminf(fminf(n.x * px[0] + n.y * py[0], n.x * px[1] + n.y * py[1]),
-                                  fminf(n.x * px[2] + n.y * py[2], n.x * px[3] + n.y * py[3]));
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {  // slot `ne`, without dynamic indexing
-            if (q == ne) { lab[q] = ab; lc[q] = fmaf(margin, kLineUnit, -low); }
-          }
-          ++ne;
-        }
+    for (int k = 0; k < PER; ++k) {
+      const unsigned w = __ballot_sync(0xffffffffu, ids_ok[k]), m = __ballot_sync(0xffffffffu, live[k] && !ids_ok[k]);
+      const unsigned below = (1u << lane) - 1u;
+      int first_w = 0, first_m = 0;
+      if (lane == 0) {
+        if (w) first_w = atomicAdd(&n_whole, __popc(w));
+        if (m) first_m = atomicAdd(&n_marks, __popc(m));
       }
+      first_w = __shfl_sync(0xffffffffu, first_w, 0);
+      first_m = __shfl_sync(0xffffffffu, first_m, 0);
+      if (ids_ok[k]) whole[first_w + __popc(w & below)] = (uint16_t)(k * kPackThreads + threadIdx.x);
+      else if (live[k]) marks[first_m + __popc(m & below)] = (uint16_t)(k * kPackThreads + threadIdx.x);
     }
-    ok = ok && (ne == 3 || ne == 4);
-    if (ne == 3) { lab[3] = lab[2]; lc[3] = lc[2]; }
-    if (!ok) {
-      const float qnan = __int_as_float(0x7fc00000);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) lc[k] = qnan;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * n_marks; i += kPackThreads)
+      records[record_at(g0 + marks[i >> 1]) + kLinesAt + (i & 1)] = make_float4(0.0f, (i & 1) ? 0.0f : never_seen(), 0.0f, 0.0f);
+    for (int first = 0; first < n_whole; first += kPackThreads) {
+      if (first + (int)threadIdx.x < n_whole) {
+        const int64_t g = g0 + whole[first + threadIdx.x];
+        build_record(r, __ldg(reinterpret_cast<const int4*>(indices) + g), vertices, cell, g, __ldg(cell + 7 * g), rcam);
+      }
+      __syncthreads();
+      const int n_rec = min(kPackThreads, n_whole - first);
+      for (int i = threadIdx.x; i < n_rec * 8; i += kPackThreads) {
+        const int row = i >> 3, k = i & 7;
+        records[record_at(g0 + whole[first + row]) + k] = sm[row * kRow + k];
+      }
+      __syncthreads();
     }
-    r[6] = make_float4(lab[0], lc[0], lab[1], lc[1]);
-    r[7] = make_float4(lab[2], lc[2], lab[3], lc[3]);
-  }
-  __syncthreads();
-  const int n_rec = (int)min((int64_t)kPackThreads, T - g0);
-  for (int i = threadIdx.x; i < n_rec * 8; i += kPackThreads) {
-    const int row = i >> 3, k = i & 7;
-    if (packed[row] == kAll || (packed[row] == kMark && k >= kLinesAt)) records[record_at(g0 + row) + k] = sm[row * kRow + k];
   }
 }
 
@@ -1552,88 +1608,111 @@ k_clear_flagged_rows(const uint8_t* __restrict__ tet_flags, int64_t T, float4* _
   }
 }
 
-// Chain rule from record gradients to vertices and cell values; one thread per tet.
-constexpr int kFinishThreads = 256;
+// Chain rule from record gradients to vertices and cell values for tets [t_begin, T).  A block looks through the flags of PER
+// tets per thread and makes a list of the flagged ones; a thread then takes one of the list.  Bound by the chain flag -> row and
+// vertex ids -> vertices and by the atomics (without them 203 of 230 us): with a list all lanes of a warp are on that chain,
+// with a thread per tet 20 of 32, and blocks of 64 threads do not wait long for their slowest warp (blocks of 256 and a thread
+// per tet: 6M tets 230 us, 18M 701, 2M 74; now 162, 484 and 62).
+constexpr int kFinishThreads = 64;
 
+template <int PER>
 __global__ void __launch_bounds__(kFinishThreads)
 k_backward_finish(const int32_t* __restrict__ indices, const float* __restrict__ vertices,
                   const float* __restrict__ cell, int64_t t_begin, int64_t T, RmCamera rcam,
                   const float4* __restrict__ grec, const uint8_t* __restrict__ tet_flags, float* __restrict__ vgrad,
                   float* __restrict__ cgrad) {
-  // the block's cell-value gradient rows (7 floats per tet) leave through shared memory as
-  // contiguous 16-byte stores
-  __shared__ __align__(16) float rows[kFinishThreads * 7];
-  const int64_t g0 = t_begin + (int64_t)blockIdx.x * kFinishThreads;  // tets [t_begin, T) are handled by this launch
-  const int64_t g = g0 + threadIdx.x;
-  float* co = rows + 7 * threadIdx.x;
-  float4 q[6];
-  bool any = false;
-  int4 id = make_int4(0, 0, 0, 0);
-  if (g < T && tet_flags[g]) {  // rows of tets without a hit were neither cleared nor written
+  constexpr int kTets = PER * kFinishThreads;
+  // the block's cell-value gradient rows (7 floats per tet, zero without a gradient) leave through shared memory as contiguous
+  // 16-byte stores
+  __shared__ __align__(16) float rows[kTets * 7];
+  __shared__ uint16_t listed[kTets];
+  __shared__ int n_listed;
+  const int64_t g0 = t_begin + (int64_t)blockIdx.x * kTets;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) n_listed = 0;
+  bool on[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int64_t g = g0 + k * kFinishThreads + threadIdx.x;
+    on[k] = g < T && tet_flags[g];
+  }
+  for (int i = threadIdx.x; i < kTets * 7 / 4; i += kFinishThreads) reinterpret_cast<float4*>(rows)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const unsigned m = __ballot_sync(0xffffffffu, on[k]);
+    int first = 0;
+    if (lane == 0 && m) first = atomicAdd(&n_listed, __popc(m));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (on[k]) listed[first + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(k * kFinishThreads + threadIdx.x);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_listed; i += kFinishThreads) {
+    const int local = listed[i];
+    const int64_t g = g0 + local;
+    float* co = rows + 7 * local;
     // the vertex ids travel with the gradient row: one dependent round trip less before the vertex gathers
-    id = __ldg(reinterpret_cast<const int4*>(indices) + g);
+    int4 id = __ldg(reinterpret_cast<const int4*>(indices) + g);
+    float4 q[6];
+    bool any = false;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       q[k] = __ldg(grec + 6 * g + k);
       any = any || q[k].x != 0.f || q[k].y != 0.f || q[k].z != 0.f || q[k].w != 0.f;
     }
-  }
-  if (!any) {
-#pragma unroll
-    for (int k = 0; k < 7; ++k) co[k] = 0.0f;
-  } else {
-  f3 cam = {__ldg(rcam.cam_pos), __ldg(rcam.cam_pos + 1), __ldg(rcam.cam_pos + 2)};
-  if (!(RM_INDEX_OK(id.x, RM_X_VERTS, 5) && RM_INDEX_OK(id.y, RM_X_VERTS, 5) && RM_INDEX_OK(id.z, RM_X_VERTS, 5) &&
-        RM_INDEX_OK(id.w, RM_X_VERTS, 5)))
-    id = make_int4(0, 0, 0, 0);
-  const int vid[4] = {id.x, id.y, id.z, id.w};
-  f3 v[4] = {load3(vertices, id.x), load3(vertices, id.y), load3(vertices, id.z), load3(vertices, id.w)};
-  PlaneSetup p;
-  make_planes(v, cam, p);
-  f3 gvv[4] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int b = i == 3 ? 1 : 0;
-    const int e1 = i < 2 ? 1 : 2;
-    const int e2 = i == 0 ? 2 : 3;
-    const float gD = q[i].w;
-    f3 g_n = {q[i].x, q[i].y, q[i].z};
-    g_n = g_n + (v[b] - cam) * (-gD);  // D = -n.(b - cam)
-    f3 g_b = p.n[i] * (-gD);
-    f3 g_raw = g_n * p.sgn[i];
-    f3 E1 = v[e1] - v[b], E2 = v[e2] - v[b];
-    f3 g_e1 = cross(E2, g_raw);
-    f3 g_e2 = cross(g_raw, E1);
-    gvv[e1] = gvv[e1] + g_e1;
-    gvv[e2] = gvv[e2] + g_e2;
-    gvv[b] = gvv[b] + g_b - g_e1 - g_e2;
-  }
-  const float* c = cell + 7 * g;
-  f3 grd = {__ldg(c + 4), __ldg(c + 5), __ldg(c + 6)};
-  const float gs0 = q[4].w;
-  f3 g_grd = {q[4].x, q[4].y, q[4].z};
-  g_grd = g_grd + (cam - v[0]) * gs0;  // s0 = grd.(cam - v0)
-  gvv[0] = gvv[0] - grd * gs0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float* vp = vgrad + 3 * (int64_t)vid[k];
-    atomicAdd(vp + 0, gvv[k].x);
-    atomicAdd(vp + 1, gvv[k].y);
-    atomicAdd(vp + 2, gvv[k].z);
-  }
-  co[0] = __ldg(c) > 0.0f ? q[5].w : 0.0f;
-  co[1] = q[5].x;
-  co[2] = q[5].y;
-  co[3] = q[5].z;
-  co[4] = g_grd.x;
-  co[5] = g_grd.y;
-  co[6] = g_grd.z;
+    if (!any) continue;
+    f3 cam = {__ldg(rcam.cam_pos), __ldg(rcam.cam_pos + 1), __ldg(rcam.cam_pos + 2)};
+    if (!(RM_INDEX_OK(id.x, RM_X_VERTS, 5) && RM_INDEX_OK(id.y, RM_X_VERTS, 5) && RM_INDEX_OK(id.z, RM_X_VERTS, 5) &&
+          RM_INDEX_OK(id.w, RM_X_VERTS, 5)))
+      id = make_int4(0, 0, 0, 0);
+    const int vid[4] = {id.x, id.y, id.z, id.w};
+    f3 v[4] = {load3(vertices, id.x), load3(vertices, id.y), load3(vertices, id.z), load3(vertices, id.w)};
+    PlaneSetup p;
+    make_planes(v, cam, p);
+    f3 gvv[4] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int b = i == 3 ? 1 : 0;
+      const int e1 = i < 2 ? 1 : 2;
+      const int e2 = i == 0 ? 2 : 3;
+      const float gD = q[i].w;
+      f3 g_n = {q[i].x, q[i].y, q[i].z};
+      g_n = g_n + (v[b] - cam) * (-gD);  // D = -n.(b - cam)
+      f3 g_b = p.n[i] * (-gD);
+      f3 g_raw = g_n * p.sgn[i];
+      f3 E1 = v[e1] - v[b], E2 = v[e2] - v[b];
+      f3 g_e1 = cross(E2, g_raw);
+      f3 g_e2 = cross(g_raw, E1);
+      gvv[e1] = gvv[e1] + g_e1;
+      gvv[e2] = gvv[e2] + g_e2;
+      gvv[b] = gvv[b] + g_b - g_e1 - g_e2;
+    }
+    const float* c = cell + 7 * g;
+    f3 grd = {__ldg(c + 4), __ldg(c + 5), __ldg(c + 6)};
+    const float gs0 = q[4].w;
+    f3 g_grd = {q[4].x, q[4].y, q[4].z};
+    g_grd = g_grd + (cam - v[0]) * gs0;  // s0 = grd.(cam - v0)
+    gvv[0] = gvv[0] - grd * gs0;
+  #pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float* vp = vgrad + 3 * (int64_t)vid[k];
+      atomicAdd(vp + 0, gvv[k].x);
+      atomicAdd(vp + 1, gvv[k].y);
+      atomicAdd(vp + 2, gvv[k].z);
+    }
+    co[0] = __ldg(c) > 0.0f ? q[5].w : 0.0f;
+    co[1] = q[5].x;
+    co[2] = q[5].y;
+    co[3] = q[5].z;
+    co[4] = g_grd.x;
+    co[5] = g_grd.y;
+    co[6] = g_grd.z;
   }
   __syncthreads();
-  const int n_rows = (int)min((int64_t)kFinishThreads, T - g0);
-  float* dst = cgrad + 7 * g0;  // 7 * 256 floats per block: 16-byte aligned whenever cgrad is
-  if (n_rows == kFinishThreads && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-    for (int i = threadIdx.x; i < kFinishThreads * 7 / 4; i += kFinishThreads)
+  const int n_rows = (int)min((int64_t)kTets, T - g0);
+  float* dst = cgrad + 7 * g0;
+  if (n_rows == kTets && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    for (int i = threadIdx.x; i < kTets * 7 / 4; i += kFinishThreads)
       reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(rows)[i];
   } else {
     for (int i = threadIdx.x; i < n_rows * 7; i += kFinishThreads) dst[i] = rows[i];
@@ -1737,14 +1816,23 @@ static inline void unit_grid(const RmCamera* cam, int* subs, int64_t* n_units, u
   *blocks = (unsigned)((*n_units + per_block - 1) / per_block);
 }
 
+// Up to a million tets a thread per tet, beyond a list per block: large meshes are scenes of which a view sees a part and 40 %
+// is empty, and they have blocks enough for a thread to look at several tets.  Packing: 13k tets 9 us (15 with a list), 600k
+// of which all have a record 43 (48), 1.8M such 111 (117), but 1M of a scene 54 (49), 2M 74 (60), 6M 299 (247), 36M 1604
+// (1345).  Chain rule: 13k 10.5 (12.6), 600k all with a gradient 56 (62), 1.8M such 160 (156), 2M of a scene 65 (62), 6M 193
+// (162), 18M 564 (484).
+constexpr int64_t kListedTets = 1000000;
+
 int rm_launch_pack(const int32_t* indices, const float* vertices, const float* cell, int64_t T, int64_t V,
                    const RmCamera* cam, const int32_t* tiles_touched, float* records, uint8_t* clear_a, uint8_t* clear_b,
                    cudaStream_t st) {
   if (T == 0) return RM_OK;
   RmProfScope prof("k_pack_records", st);
-  RM_CUDA_CHECK(rm_launch(rm::k_pack_records, (unsigned)((T + rm::kPackThreads - 1) / rm::kPackThreads), rm::kPackThreads,
-                          0, st, indices, vertices, cell, T, V, *cam, tiles_touched, reinterpret_cast<float4*>(records),
-                          clear_a, clear_b));
+  const int per = T > kListedTets ? 3 : 1;
+  auto kernel = per == 3 ? rm::k_pack_records<3> : rm::k_pack_records<1>;
+  const int64_t per_block = (int64_t)per * rm::kPackThreads;
+  RM_CUDA_CHECK(rm_launch(kernel, (unsigned)((T + per_block - 1) / per_block), rm::kPackThreads, 0, st, indices, vertices, cell, T, V, *cam,
+                          tiles_touched, reinterpret_cast<float4*>(records), clear_a, clear_b));
   return RM_OK;
 }
 
@@ -1910,10 +1998,12 @@ int rm_launch_backward_finish(const int32_t* indices, const float* vertices, con
                               float* vgrad, float* cgrad, cudaStream_t st) {
   if (t_end <= t_begin) return RM_OK;
   RmProfScope prof("k_backward_finish", st);
-  RM_CUDA_CHECK(rm_launch(rm::k_backward_finish,
-                          (unsigned)((t_end - t_begin + rm::kFinishThreads - 1) / rm::kFinishThreads), rm::kFinishThreads, 0, st,
-                          indices, vertices, cell, t_begin, t_end, *cam, reinterpret_cast<const float4*>(grec),
-                          hits->tet_flags, vgrad, cgrad));
+  const int64_t n = t_end - t_begin;
+  const int per = n > kListedTets ? 4 : 1;
+  auto kernel = per == 4 ? rm::k_backward_finish<4> : rm::k_backward_finish<1>;
+  const int64_t per_block = (int64_t)per * rm::kFinishThreads;
+  RM_CUDA_CHECK(rm_launch(kernel, (unsigned)((n + per_block - 1) / per_block), rm::kFinishThreads, 0, st, indices, vertices, cell,
+                          t_begin, t_end, *cam, reinterpret_cast<const float4*>(grec), hits->tet_flags, vgrad, cgrad));
   return RM_OK;
 }
 
@@ -1980,11 +2070,8 @@ extern "C" int rm_backward_static_scratch(const int32_t* sorted_tetra_idx, const
   rc = launch_backward_walk(tile_ranges, records, cam, ray_jitter, output_img, distortion_img, hits, grad_output_img,
                             grad_distortion_img, scratch, n_tets, st);
   if (rc) return rc;
-  RmProfScope prof2("k_backward_finish", st);
-  RM_CUDA_CHECK(rm_launch(rm::k_backward_finish, (unsigned)((n_tets + rm::kFinishThreads - 1) / rm::kFinishThreads),
-                          rm::kFinishThreads, 0, st, indices, vertices, cell_values, 0, n_tets, *cam,
-                          reinterpret_cast<const float4*>(scratch), hits->tet_flags, vertices_grad, cell_values_grad));
-  return RM_OK;
+  return rm_launch_backward_finish(indices, vertices, cell_values, 0, n_tets, cam, scratch, hits, vertices_grad, cell_values_grad,
+                                   st);
 }
 
 // Bounds-checked build: extents of the caller-owned arrays of the integration stages (the entry points
