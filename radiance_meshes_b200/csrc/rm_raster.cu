@@ -1154,9 +1154,13 @@ __device__ __forceinline__ void walk_unit(
   }
 }
 
-// Units by halves or by pairs.
+// Units by halves or by pairs.  A block holds its place until its last warp is done: two warps where units are long and many
+// (statistics, 2M tets: 2590 us with four, 2566 with two, 2563 with one), four where neighbouring units that share records
+// count (600k tets, 800 x 800, pairs: 416 us with four, 435 with two, 469 with one).
+template <ForwardMode MODE>
+constexpr int kFwdWarps = MODE == kStats ? 2 : kWarpsPerBlock;
 template <ForwardMode MODE, bool PAIR>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, MODE == kStats ? 4 : 5)
+__global__ void __launch_bounds__(kFwdWarps<MODE> * 32, (MODE == kStats ? 16 : 20) / kFwdWarps<MODE>)
 k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
           const float2* __restrict__ jitter, float4* __restrict__ out_img, float* __restrict__ dist_img,
           int32_t* __restrict__ n_contrib, int32_t* __restrict__ hit_counts, int32_t* __restrict__ hit_ids,
@@ -1164,14 +1168,16 @@ k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, con
           float ladder_p, StatsArgs stats) {
   extern __shared__ __align__(16) unsigned char smem_fwd[];
   const int warp = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
-  const int64_t at = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
+  const int64_t at = (int64_t)blockIdx.x * kFwdWarps<MODE> + warp;
   walk_unit<MODE, PAIR>(reinterpret_cast<ForwardShared<MODE>*>(smem_fwd)[warp], PAIR ? at : 2 * at + half, INT_MAX, list, ranges,
                         records, rcam, jitter, out_img, dist_img, n_contrib, hit_counts, hit_ids, hit_masks, tet_flags, subs,
                         n_units, pre_multi, ladder_p, stats);
 }
 
 // Long first: the first `long_blocks` of the grid take the tiles whose list is longer than `long_list`.
-// 92 registers, as the walk by halves takes in a kernel of its own.
+// 92 registers, as the walk by halves takes in a kernel of its own.  Two warps per block: the same time at 2M tets, with four
+// 6M 1874 us in place of 1857, 18M 2557 in place of 2514.
+constexpr int kLongFirstWarps = 2;
 __global__ void __maxnreg__(92)
 k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
                      const float2* __restrict__ jitter, float4* __restrict__ out_img, float* __restrict__ dist_img,
@@ -1183,8 +1189,8 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
   FwdShared& sm = reinterpret_cast<FwdShared*>(smem_fwd)[warp];
   // Warp w of the first blocks looks through units w, w + walkers, ..., 32 at a time: the tiles of a region with long lists
   // go to different warps.
-  const int64_t walkers = (int64_t)long_blocks * kWarpsPerBlock;
-  int64_t at = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
+  const int64_t walkers = (int64_t)long_blocks * kLongFirstWarps;
+  int64_t at = (int64_t)blockIdx.x * kLongFirstWarps + warp;
   if (at < walkers) {
     const int first = rcam.tile_row_begin * rcam.grid_width;
     for (; at < n_units; at += 32 * walkers) {
@@ -1201,7 +1207,7 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
     }
     return;
   }
-  at = (int64_t)(blockIdx.x - (unsigned)long_blocks) * kWarpsPerBlock + warp;
+  at = (int64_t)(blockIdx.x - (unsigned)long_blocks) * kLongFirstWarps + warp;
   walk_unit<kColor, false>(sm, at * 2 + (lane >> 4), long_list, list, ranges, records, rcam, jitter, out_img, dist_img, n_contrib,
                            hit_counts, hit_ids, hit_masks, tet_flags, subs, n_units, 0.0f, 0.0f, StatsArgs{});
 }
@@ -1805,12 +1811,12 @@ int rm_launch_distortion_loss_backward(const float* dist, int64_t n, const float
 // ----------------------------------------------------------------------------
 // host-side launchers used by rm_api.cu
 // ----------------------------------------------------------------------------
-static inline void unit_grid(const RmCamera* cam, int* subs, int64_t* n_units, unsigned* blocks) {
+static inline void unit_grid(const RmCamera* cam, int warps, int* subs, int64_t* n_units, unsigned* blocks) {
   int px = cam->tile_width * cam->tile_height;
   *subs = (px + 15) / 16;
   int64_t tiles = (int64_t)(cam->tile_row_end - cam->tile_row_begin) * cam->grid_width;
   *n_units = tiles * *subs;
-  int64_t per_block = rm::kWarpsPerBlock * 2;
+  int64_t per_block = warps * 2;
   *blocks = (unsigned)((*n_units + per_block - 1) / per_block);
 }
 
@@ -1842,7 +1848,7 @@ int rm_launch_pack(const int32_t* indices, const float* vertices, const float* c
 //              57 us in place of 64 on 400 x 400 pixels, but 95 in place of 84 on 560 x 560).
 //   more:      long first, a long list being one of three times the average.  Up to five times the result is the
 //              same within 1 %; at 1.5, pairs take over so much of the work that its overhead shows.
-constexpr int64_t kWave = 148 * 5 * rm::kWarpsPerBlock * 2;
+constexpr int64_t kWave = 148 * 20 * 2;
 static bool deal_by_pairs(int64_t n_units, int64_t tiles, int64_t n_list) {
   return n_units <= 2 * kWave || (n_units <= 8 * kWave && n_list >= 64 * tiles);
 }
@@ -1853,7 +1859,7 @@ int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* r
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, &subs, &n_units, &blocks);
+  unit_grid(cam, rm::kWarpsPerBlock, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
   const int64_t tiles = n_units / subs;
   const unsigned pair_blocks = (unsigned)((n_units + rm::kWarpsPerBlock - 1) / rm::kWarpsPerBlock);
@@ -1866,8 +1872,10 @@ int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* r
   const RmHitList h = hits ? *hits : RmHitList{nullptr, nullptr, nullptr, nullptr};
   RmProfScope prof("k_forward", st);
   if (n_units > 8 * kWave && n_list >= 0) {
-    const int long_blocks = 148 * 5, long_list = (int)std::min<int64_t>(3 * n_list / tiles, INT_MAX);
-    RM_CUDA_CHECK(rm_launch(rm::k_forward_long_first, blocks + long_blocks, threads, smem, st, list, tiles_list, recs, *cam,
+    constexpr int warps = rm::kLongFirstWarps, long_blocks = 148 * 20 / warps;
+    const int long_list = (int)std::min<int64_t>(3 * n_list / tiles, INT_MAX);
+    blocks = (unsigned)((n_units + 2 * warps - 1) / (2 * warps));
+    RM_CUDA_CHECK(rm_launch(rm::k_forward_long_first, blocks + long_blocks, warps * 32, warps * sizeof(rm::FwdShared), st, list, tiles_list, recs, *cam,
                             jit, img, dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, long_list,
                             long_blocks));
   } else {
@@ -1886,7 +1894,7 @@ int rm_launch_forward_constant_color(const int32_t* list, const int32_t* ranges,
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, &subs, &n_units, &blocks);
+  unit_grid(cam, rm::kWarpsPerBlock, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
   RmProfScope prof("k_forward<constant colour>", st);
   const bool pair = deal_by_pairs(n_units, n_units / subs, n_list);
@@ -1912,7 +1920,7 @@ int rm_launch_backward_constant_color(const int32_t* list, const int32_t* ranges
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, &subs, &n_units, &blocks);
+  unit_grid(cam, rm::kWarpsPerBlock, &subs, &n_units, &blocks);
   if (n_units > 0) {
     RmProfScope prof("k_backward<constant colour>", st);
     RM_CUDA_CHECK(rm_launch(rm::k_backward_cc, blocks, rm::kWarpsPerBlock * 32, 0, st, list,
@@ -1933,13 +1941,14 @@ int rm_launch_tet_err(const int32_t* list, const int32_t* ranges, const float* r
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, &subs, &n_units, &blocks);
+  constexpr int warps = rm::kFwdWarps<rm::kStats>;
+  unit_grid(cam, warps, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
-  constexpr size_t smem = rm::kWarpsPerBlock * sizeof(rm::StatsShared);
+  constexpr size_t smem = warps * sizeof(rm::StatsShared);
   RM_CUDA_CHECK(cudaFuncSetAttribute(rm::k_forward<rm::kStats, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   RmProfScope prof("k_tet_err", st);
-  RM_CUDA_CHECK(rm_launch(rm::k_forward<rm::kStats, false>, blocks, rm::kWarpsPerBlock * 32, smem, st, list,
+  RM_CUDA_CHECK(rm_launch(rm::k_forward<rm::kStats, false>, blocks, warps * 32, smem, st, list,
                           reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
                           nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, subs, n_units, 0.0f, 0.0f,
                           rm::StatsArgs{pixel_err, ssim_err, tet_err, tet_count}));
@@ -1952,7 +1961,7 @@ static int launch_backward_walk(const int32_t* ranges, const float* records, con
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, &subs, &n_units, &blocks);
+  unit_grid(cam, rm::kWarpsPerBlock, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
   constexpr size_t smem = rm::kWarpsPerBlock * sizeof(rm::BwdShared);
   // up to two waves of half-warps the longest hit lists set the time; beyond, the shuffles' cost shows (2M tets, 400 x 400:
