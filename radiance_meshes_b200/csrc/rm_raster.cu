@@ -1275,8 +1275,13 @@ struct BwdShared {                                // 11.1 KB: five blocks of fou
 // PAIR: one unit per warp, 16 entries a round and two lanes per pixel, each on every other entry of the pixel, the last
 // first; what the two entries change of the state is handed over by shuffles.  Both phases then take half as many rounds in
 // a row (13k tets, 128 x 128: 70 -> 49 us; 60k, 203 x 317: 154 -> 123 us; 2M, 300 x 300: 543 -> 459 us).
+// On its small grids a block of one warp: units of uneven length then do not hold each other's places (13k tets, 128 x 128:
+// 51.6 us with four, 47.6 with one; 2M of a scene, 300 x 300: 440 and 365).  Large grids lose by it what neighbouring units
+// share (6M: 2202 us with four, 2245 with one).
 template <bool PAIR>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
+constexpr int kBwdWarps = PAIR ? 1 : kWarpsPerBlock;
+template <bool PAIR>
+__global__ void __launch_bounds__(kBwdWarps<PAIR> * 32, 20 / kBwdWarps<PAIR>)
 k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
            const float2* __restrict__ jitter, const float4* __restrict__ out_img, const float* __restrict__ dist_img,
            const int32_t* __restrict__ hit_counts, const int32_t* __restrict__ hit_ids,
@@ -1292,7 +1297,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   BwdShared& sm = reinterpret_cast<BwdShared*>(smem_bwd)[warp];
   float4* const staged = sm.stage + half * kBwdBatch * kBwdStageStride;
   float4 *const planes = sm.planes + half * kBwdBatch * 16, *const fields = sm.fields + half * kBwdBatch * 16;
-  const int64_t unit = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * (PAIR ? 1 : 2) + half;
+  const int64_t unit = ((int64_t)blockIdx.x * kBwdWarps<PAIR> + warp) * (PAIR ? 1 : 2) + half;
   Unit u = make_unit(rcam, ranges, unit, n_units, subs, lane16);
 
   f3 d = {0.f, 0.f, 1.f};
@@ -1992,17 +1997,18 @@ static int launch_backward_walk(const int32_t* ranges, const float* records, con
   int subs;
   int64_t n_units;
   unsigned blocks;
-  unit_grid(cam, rm::kWarpsPerBlock, &subs, &n_units, &blocks);
+  unit_grid(cam, rm::kBwdWarps<false>, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
-  constexpr size_t smem = rm::kWarpsPerBlock * sizeof(rm::BwdShared);
   // up to two waves of half-warps the longest hit lists set the time; beyond, the shuffles' cost shows (2M tets, 400 x 400:
   // 683 -> 662 us, 560 x 560: 1039 -> 1092 us)
   const bool pair = n_units <= 2 * kWave;
-  if (pair) blocks = (unsigned)((n_units + rm::kWarpsPerBlock - 1) / rm::kWarpsPerBlock);
+  const int warps = pair ? rm::kBwdWarps<true> : rm::kBwdWarps<false>;
+  if (pair) blocks = (unsigned)((n_units + warps - 1) / warps);
+  const size_t smem = warps * sizeof(rm::BwdShared);
   auto kernel = pair ? rm::k_backward<true> : rm::k_backward<false>;
   RM_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   RmProfScope prof("k_backward", st);
-  RM_CUDA_CHECK(rm_launch_behind(T, kernel, blocks, rm::kWarpsPerBlock * 32, smem, st,
+  RM_CUDA_CHECK(rm_launch_behind(T, kernel, blocks, warps * 32, smem, st,
                                  reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam,
                                  reinterpret_cast<const float2*>(jitter), reinterpret_cast<const float4*>(out_img), dist_img,
                                  hits->counts, hits->ids, hits->masks, reinterpret_cast<const float4*>(g_img), g_dist, grec,
