@@ -519,12 +519,13 @@ __device__ __forceinline__ void add_coverage(const ProjectOut& o, const DevCam& 
   }
 }
 
-// One thread per tet (and, for the NaN scan, per vertex coordinate).  Bound by instruction issue (6M tets: 70 % of the slots;
-// no block barriers, or persistent warps that fetch vertices ahead, are no faster).  The camera sits in shared memory (32 loads per thread from global before), a warp's depths and circumcentres
-// leave through shared memory as 16-byte stores, and the reference's exact arithmetic is left to k_project_deferred, for
-// the tets whose rectangle an estimate does not decide: a few lanes of a warp would hold up the rest for thousands of
-// instructions.  With the exact sequence for every tet 6M tets, 1080p took 369 us, with the deferral 290 (238 now, see
-// add_coverage); 1M through a fisheye 436 us with the deferred tets done in place, 81 with the deferral (59 now).
+// One thread per tet (and, for the NaN scan, per vertex coordinate).  Bound by instruction issue (6M tets: 70 % of the
+// slots; no block barriers, or persistent warps that fetch vertices ahead, are no faster).  The camera sits in shared memory
+// (32 loads per thread from global before), a warp's depths and circumcentres leave through shared memory as 16-byte stores,
+// and the reference's exact arithmetic is left to k_project_deferred, for the tets whose rectangle an estimate does not
+// decide: a few lanes of a warp would hold up the rest for thousands of instructions.  With the exact sequence for every tet
+// 6M tets, 1080p took 369 us, with the deferral 290 (238 now, see add_coverage); 1M through a fisheye 436 us with the
+// deferred tets done in place, 81 with the deferral (59 now).
 constexpr int kProjectThreads = 128;
 
 template <bool FISHEYE>
