@@ -513,19 +513,19 @@ __device__ __forceinline__ Crossing slab_planes(const float4 (&rec)[4], const Ra
 // Weights of the closed-form segment integral for optical depth x > 0:
 //   alpha = exp(-x), phi = (1 - alpha)/x, w0 = phi - alpha, w1 = 1 - phi, and slope = w0/x = -d phi/dx.
 // Below x = 0.25 the differences cancel: w1 = x p(x) comes from its Taylor series (truncation < 1e-7 relative) and
-// w0 from w0 + w1 = 1 - alpha = x phi = x - x w1, a difference that halves the leading term only; above, from the
-// fast exponential.
-__device__ __forceinline__ void segment_weights(float x, float& alpha, float& w, float& w0, float& w1, float& slope) {
+// w0 from w0 + w1 = 1 - alpha = x phi = x - x w1, a difference that halves the leading term only; above, both come from the
+// fast exponential, each by a multiply-add of its own: w0 falls as 1/x, and as a difference of the sum and w1, two numbers
+// near 1, it would lose all precision to an optical depth of 1e7.
+__device__ __forceinline__ void segment_weights(float x, float& alpha, float& w0, float& w1, float& slope) {
   alpha = fast_exp(-x);
   // p = 1/2 - x/6 + x^2/24 - x^3/120 + x^4/720 - x^5/5040
   const float p = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 5040.0f, 1.0f / 720.0f), -1.0f / 120.0f), 1.0f / 24.0f),
                                -1.0f / 6.0f), 0.5f);
-  const float inv = fast_rcp(x), series = __fmul_rn(x, p);
+  const float inv = fast_rcp(x), rest = 1.0f - alpha, series = __fmul_rn(x, p);
   // both forms are evaluated: the lanes of a warp nearly always need both, and selects cost less than the branch
   const bool thin = x < 0.25f;
-  w = thin ? fmaf(-x, series, x) : 1.0f - alpha;
-  w1 = thin ? series : fmaf(-w, inv, 1.0f);
-  w0 = w - w1;
+  w1 = thin ? series : fmaf(-rest, inv, 1.0f);
+  w0 = thin ? fmaf(-x, series, x) - series : fmaf(rest, inv, -alpha);
   slope = thin ? (1.0f - w1) - p : w0 * inv;
 }
 
@@ -534,10 +534,10 @@ __device__ __forceinline__ void segment_weights(float x, float& alpha, float& w,
 __device__ __forceinline__ void integrate(float4 cg, float4 cb, f3 d, float min_t, Eval& e) {
   const float gd = dot_fma({cg.x, cg.y, cg.z}, d);
   const float oe = fmaf(e.enter + min_t, gd, cg.w), ox = fmaf(e.exit + min_t, gd, cg.w);
-  float w, w0, w1, slope;
-  segment_weights(e.tau, e.alpha, w, w0, w1, slope);
+  float w0, w1, slope;
+  segment_weights(e.tau, e.alpha, w0, w1, slope);
   // w0 (base + ox) + w1 (base + oe), channel by channel: the gradient is the same on all of them
-  const float o = fmaf(w0, ox, w1 * oe);
+  const float w = w0 + w1, o = fmaf(w0, ox, w1 * oe);
   e.cr = fmaf(w, cb.x, o);
   e.cg = fmaf(w, cb.y, o);
   e.cb = fmaf(w, cb.z, o);
@@ -1414,9 +1414,9 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
         const float X = exit + min_t, E = enter + min_t;
         const float gd = cg.x * d.x + cg.y * d.y + cg.z * d.z;
         const float oe = fmaf(E, gd, cg.w), ox = fmaf(X, gd, cg.w);
-        float alpha = 0.f, w = 0.f, w0 = 0.f, w1 = 0.f, slope = 0.f;
-        if (hit) segment_weights(tau, alpha, w, w0, w1, slope);
-        const float gcb = gr * cb.x + gg * cb.y + gb * cb.z;
+        float alpha = 0.f, w0 = 0.f, w1 = 0.f, slope = 0.f;
+        if (hit) segment_weights(tau, alpha, w0, w1, slope);
+        const float w = w0 + w1, gcb = gr * cb.x + gg * cb.y + gb * cb.z;
         const float up = hit ? fmaf(w, gcb, fmaf(w0, ox, w1 * oe) * G) * Tp : 0.0f;
         const float o_up = __shfl_xor_sync(FULL, up, 16), glogT1 = glogT + (second ? o_up : up);
         if (hit) {
@@ -1461,8 +1461,8 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
         const float X = exit + min_t, E = enter + min_t;
         const float gd = cg.x * d.x + cg.y * d.y + cg.z * d.z;
         const float oe = fmaf(E, gd, cg.w), ox = fmaf(X, gd, cg.w);
-        float alpha, w, w0, w1, slope;
-        segment_weights(tau, alpha, w, w0, w1, slope);
+        float alpha, w0, w1, slope;
+        segment_weights(tau, alpha, w0, w1, slope);
         // undo: state before this tet
         logT += tau;
         const float Tp = fast_exp(fminf(logT, 46.0517f));
@@ -1471,6 +1471,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
         sw -= m1;
         // reverse of the state update
         const float g_m1 = fmaf(sz, gx2, gw), g_m0 = fmaf(sw, gy2, gz);
+        const float w = w0 + w1;
         const float gcb = gr * cb.x + gg * cb.y + gb * cb.z;  // colour of the tet against the upstream gradient
         const float g_a = -glogT;
         glogT = fmaf(fmaf(w, gcb, fmaf(w0, ox, w1 * oe) * G), Tp, glogT);
