@@ -207,13 +207,13 @@ __device__ __forceinline__ void build_record(float4* r, int4 id, const float* __
   r[7] = make_float4(lab[2], lc[2], lab[3], lc[3]);
 }
 
-// A thread builds one record in registers; the block then writes its records through shared memory, so that the global stores
-// are contiguous.  What of a record is written: nothing for a culled tet, which appears in no list; the lines' sector for a
-// tet of zero density (a mark), which the integration kernels drop by its first line without reading more (40 % of the tets of
-// an unbounded scene); else all of it.
-// PER = 1: a thread per tet.  PER > 1: the block first looks at PER tets per thread and makes lists of those to be written
-// whole and of those to be marked, so that all lanes of a warp have a record to build (of 6M tets 46 % have one: 19 lanes of 32
-// had something to do, now 25).
+// A thread builds one record in registers; it is then written through shared memory, so that the global stores are contiguous.
+// What of a record is written: nothing for a culled tet, which appears in no list; the lines' sector for a tet of zero density
+// (a mark), which the integration kernels drop by its first line without reading more (40 % of the tets of an unbounded scene);
+// else all of it.
+// PER = 1: a thread per tet.  PER > 1: the block first looks at PER tets per thread and lists those to be written whole; each of
+// its warps then takes 32 of the list at a time, so that all lanes have a record to build and no warp waits for another one (of
+// 6M tets 46 % have one, by runs: a list per warp leaves its last round half empty, 256 us in place of 236).
 template <int PER>
 __global__ void __launch_bounds__(kPackThreads, 8)
 k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ vertices,
@@ -223,12 +223,12 @@ k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ ve
   constexpr int kRow = 9;  // 8 used; the odd stride spreads the rows over the banks
   constexpr int kTets = PER * kPackThreads;
   __shared__ __align__(16) float4 sm[kPackThreads * kRow];
-  __shared__ uint16_t whole[kTets], marks[kTets];
-  __shared__ int n_whole, n_marks;
+  __shared__ uint16_t list[kTets];  // PER = 1: what of the thread's record is written
+  __shared__ int n_listed;
   const int64_t g0 = (int64_t)blockIdx.x * kTets;
-  const int lane = threadIdx.x & 31;
-  float4* r = sm + threadIdx.x * kRow;
-  if (PER > 1 && threadIdx.x == 0) n_whole = n_marks = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float4* const rows = sm + 32 * warp * kRow;
+  if (PER > 1 && threadIdx.x == 0) n_listed = 0;
   bool live[PER], ids_ok[PER];
   float density[PER];
   int4 id[PER];
@@ -256,7 +256,8 @@ k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ ve
   if constexpr (PER == 1) {
     enum { kNone, kMark, kAll };
     const int64_t g = g0 + threadIdx.x;
-    whole[threadIdx.x] = !live[0] ? kNone : ids_ok[0] ? kAll : kMark;
+    float4* r = sm + threadIdx.x * kRow;
+    list[threadIdx.x] = !live[0] ? kNone : ids_ok[0] ? kAll : kMark;
     r[6] = make_float4(0.0f, never_seen(), 0.0f, 0.0f);
     r[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (ids_ok[0]) build_record(r, id[0], vertices, cell, g, density[0], rcam);
@@ -264,40 +265,46 @@ k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ ve
     const int n_rec = (int)min((int64_t)kPackThreads, T - g0);
     for (int i = threadIdx.x; i < n_rec * 8; i += kPackThreads) {
       const int row = i >> 3, k = i & 7;
-      if (whole[row] == kAll || (whole[row] == kMark && k >= kLinesAt)) records[record_at(g0 + row) + k] = sm[row * kRow + k];
+      if (list[row] == kAll || (list[row] == kMark && k >= kLinesAt)) records[record_at(g0 + row) + k] = sm[row * kRow + k];
     }
-  } else {
-    __syncthreads();
+    return;
+  }
+  __syncthreads();
+  {
+    unsigned w[PER];
+    int n = 0, first = 0;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
-      const unsigned w = __ballot_sync(0xffffffffu, ids_ok[k]), m = __ballot_sync(0xffffffffu, live[k] && !ids_ok[k]);
-      const unsigned below = (1u << lane) - 1u;
-      int first_w = 0, first_m = 0;
-      if (lane == 0) {
-        if (w) first_w = atomicAdd(&n_whole, __popc(w));
-        if (m) first_m = atomicAdd(&n_marks, __popc(m));
-      }
-      first_w = __shfl_sync(0xffffffffu, first_w, 0);
-      first_m = __shfl_sync(0xffffffffu, first_m, 0);
-      if (ids_ok[k]) whole[first_w + __popc(w & below)] = (uint16_t)(k * kPackThreads + threadIdx.x);
-      else if (live[k]) marks[first_m + __popc(m & below)] = (uint16_t)(k * kPackThreads + threadIdx.x);
+      w[k] = __ballot_sync(0xffffffffu, ids_ok[k]);
+      n += __popc(w[k]);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 2 * n_marks; i += kPackThreads)
-      records[record_at(g0 + marks[i >> 1]) + kLinesAt + (i & 1)] = make_float4(0.0f, (i & 1) ? 0.0f : never_seen(), 0.0f, 0.0f);
-    for (int first = 0; first < n_whole; first += kPackThreads) {
-      if (first + (int)threadIdx.x < n_whole) {
-        const int64_t g = g0 + whole[first + threadIdx.x];
-        build_record(r, __ldg(reinterpret_cast<const int4*>(indices) + g), vertices, cell, g, __ldg(cell + 7 * g), rcam);
+    if (lane == 0 && n) first = atomicAdd(&n_listed, n);
+    first = __shfl_sync(0xffffffffu, first, 0);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      if (ids_ok[k]) list[first + __popc(w[k] & ((1u << lane) - 1u))] = (uint16_t)(k * kPackThreads + threadIdx.x);
+      first += __popc(w[k]);
+      if (live[k] && !ids_ok[k]) {
+        float4* const lines = records + record_at(g0 + k * kPackThreads + threadIdx.x) + kLinesAt;
+        lines[0] = make_float4(0.0f, never_seen(), 0.0f, 0.0f);
+        lines[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
-      __syncthreads();
-      const int n_rec = min(kPackThreads, n_whole - first);
-      for (int i = threadIdx.x; i < n_rec * 8; i += kPackThreads) {
-        const int row = i >> 3, k = i & 7;
-        records[record_at(g0 + whole[first + row]) + k] = sm[row * kRow + k];
-      }
-      __syncthreads();
     }
+  }
+  __syncthreads();
+  const int n = n_listed;
+  for (int first = 32 * warp; first < n; first += kPackThreads) {
+    if (first + lane < n) {
+      const int64_t g = g0 + list[first + lane];
+      build_record(rows + lane * kRow, __ldg(reinterpret_cast<const int4*>(indices) + g), vertices, cell, g, __ldg(cell + 7 * g), rcam);
+    }
+    __syncwarp();
+    const int n_rec = min(32, n - first);
+    for (int i = lane; i < n_rec * 8; i += 32) {
+      const int row = i >> 3, k = i & 7;
+      records[record_at(g0 + list[first + row]) + k] = rows[row * kRow + k];
+    }
+    __syncwarp();
   }
 }
 
@@ -1861,11 +1868,12 @@ static inline void unit_grid(const RmCamera* cam, int warps, int* subs, int64_t*
   *blocks = (unsigned)((*n_units + per_block - 1) / per_block);
 }
 
-// Up to a million tets a thread per tet, beyond a list per block: large meshes are scenes of which a view sees a part and 40 %
-// is empty, and they have blocks enough for a thread to look at several tets.  Packing: 13k tets 9 us (15 with a list), 600k
-// of which all have a record 43 (48), 1.8M such 111 (117), but 1M of a scene 54 (49), 2M 74 (60), 6M 299 (247), 36M 1604
-// (1345).  Chain rule: 13k 10.5 (12.6), 600k all with a gradient 56 (62), 1.8M such 160 (156), 2M of a scene 65 (62), 6M 193
-// (162), 18M 564 (484).
+// Up to a million tets a thread per tet, beyond several: large meshes are scenes of which a view sees a part and 40 % is empty,
+// and they have blocks enough for a thread to look at several tets.  Packing with a thread per tet (with lists): 13k tets 8.5 us
+// (15), scenes of 2M 77 (60), 6.7M 300 (236), 21M 937 (735), the last two in random order 330 (275), 1054 (961).  Meshes that
+// have a record of every tet lose little by it: 0.6M 43 (47), 1.05M 64 (68), 2M 111 (112), 6.7M 364 (349).
+// Chain rule: 13k 10.5 (12.6), 600k all with a gradient 56 (62), 1.8M such 160 (156), 2M of a scene 65 (62), 6M 193 (162), 18M
+// 564 (484).
 constexpr int64_t kListedTets = 1000000;
 
 int rm_launch_pack(const int32_t* indices, const float* vertices, const float* cell, int64_t T, int64_t V,
