@@ -1660,11 +1660,12 @@ k_clear_flagged_rows(const uint8_t* __restrict__ tet_flags, int64_t T, float4* _
   }
 }
 
-// Chain rule from record gradients to vertices and cell values for tets [t_begin, T).  A block looks through the flags of PER
-// tets per thread and makes a list of the flagged ones; a thread then takes one of the list.  Bound by the chain flag -> row and
-// vertex ids -> vertices and by the atomics (without them 203 of 230 us): with a list all lanes of a warp are on that chain,
-// with a thread per tet 20 of 32, and blocks of 64 threads do not wait long for their slowest warp (blocks of 256 and a thread
-// per tet: 6M tets 230 us, 18M 701, 2M 74; now 162, 484 and 62).
+// Chain rule from record gradients to vertices and cell values for tets [t_begin, T).  A warp looks through the flags of PER
+// tets per lane and lists the flagged ones; a lane then takes one of the list.  Bound by the chain flag -> row and vertex ids ->
+// vertices and by the atomics, on which all lanes of a warp are with a list, 20 of 32 with a tet per lane.  Warps wait for
+// nobody: a list and rows of the whole block of 64 threads, PER = 4, cost meshes with a gradient in every tet more than a
+// thread per tet did (1.05M 92.5 us -> 94.5, 2M in random order 168 -> 175; now 90.5 and 171).  Scenes with a thread per tet in
+// blocks of 256: 2M 78 us, 6.7M 252, 21M 595; now 62, 187 and 353.
 constexpr int kFinishThreads = 64;
 
 template <int PER>
@@ -1673,34 +1674,32 @@ k_backward_finish(const int32_t* __restrict__ indices, const float* __restrict__
                   const float* __restrict__ cell, int64_t t_begin, int64_t T, RmCamera rcam,
                   const float4* __restrict__ grec, const uint8_t* __restrict__ tet_flags, float* __restrict__ vgrad,
                   float* __restrict__ cgrad) {
-  constexpr int kTets = PER * kFinishThreads;
-  // the block's cell-value gradient rows (7 floats per tet, zero without a gradient) leave through shared memory as contiguous
-  // 16-byte stores
-  __shared__ __align__(16) float rows[kTets * 7];
-  __shared__ uint16_t listed[kTets];
-  __shared__ int n_listed;
-  const int64_t g0 = t_begin + (int64_t)blockIdx.x * kTets;
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) n_listed = 0;
+  // the cell-value gradient rows of a warp's tets (7 floats per tet, zero without a gradient) leave through shared memory as
+  // contiguous 16-byte stores
+  constexpr int kTets = 32 * PER;
+  __shared__ __align__(16) float all_rows[kFinishThreads * PER * 7];
+  __shared__ uint8_t lists[kFinishThreads * PER];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t g0 = t_begin + ((int64_t)blockIdx.x * kFinishThreads + 32 * warp) * PER;
+  float* const rows = all_rows + warp * kTets * 7;
+  uint8_t* const list = lists + warp * kTets;
   bool on[PER];
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
-    const int64_t g = g0 + k * kFinishThreads + threadIdx.x;
+    const int64_t g = g0 + 32 * k + lane;
     on[k] = g < T && tet_flags[g];
   }
-  for (int i = threadIdx.x; i < kTets * 7 / 4; i += kFinishThreads) reinterpret_cast<float4*>(rows)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
+  for (int i = lane; i < kTets * 7 / 4; i += 32) reinterpret_cast<float4*>(rows)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  int n = 0;
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
     const unsigned m = __ballot_sync(0xffffffffu, on[k]);
-    int first = 0;
-    if (lane == 0 && m) first = atomicAdd(&n_listed, __popc(m));
-    first = __shfl_sync(0xffffffffu, first, 0);
-    if (on[k]) listed[first + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(k * kFinishThreads + threadIdx.x);
+    if (on[k]) list[n + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
+    n += __popc(m);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_listed; i += kFinishThreads) {
-    const int local = listed[i];
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    const int local = list[i];
     const int64_t g = g0 + local;
     float* co = rows + 7 * local;
     // the vertex ids travel with the gradient row: one dependent round trip less before the vertex gathers
@@ -1760,14 +1759,14 @@ k_backward_finish(const int32_t* __restrict__ indices, const float* __restrict__
     co[5] = g_grd.y;
     co[6] = g_grd.z;
   }
-  __syncthreads();
+  __syncwarp();
   const int n_rows = (int)min((int64_t)kTets, T - g0);
   float* dst = cgrad + 7 * g0;
   if (n_rows == kTets && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-    for (int i = threadIdx.x; i < kTets * 7 / 4; i += kFinishThreads)
+    for (int i = lane; i < kTets * 7 / 4; i += 32)
       reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(rows)[i];
   } else {
-    for (int i = threadIdx.x; i < n_rows * 7; i += kFinishThreads) dst[i] = rows[i];
+    for (int i = lane; i < n_rows * 7; i += 32) dst[i] = rows[i];
   }
 }
 
@@ -1872,8 +1871,8 @@ static inline void unit_grid(const RmCamera* cam, int warps, int* subs, int64_t*
 // and they have blocks enough for a thread to look at several tets.  Packing with a thread per tet (with lists): 13k tets 8.5 us
 // (15), scenes of 2M 77 (60), 6.7M 300 (236), 21M 937 (735), the last two in random order 330 (275), 1054 (961).  Meshes that
 // have a record of every tet lose little by it: 0.6M 43 (47), 1.05M 64 (68), 2M 111 (112), 6.7M 364 (349).
-// Chain rule: 13k 10.5 (12.6), 600k all with a gradient 56 (62), 1.8M such 160 (156), 2M of a scene 65 (62), 6M 193 (162), 18M
-// 564 (484).
+// Chain rule: 0.6M all with a gradient 57.7 (59.8), 1.05M such 90.4 (90.6), 2M such 158 (156), 6.7M such 514 (501), scenes of
+// 0.6M 23 (25), 2M 62 (62), 6.7M 195 (187), 21M 385 (353).
 constexpr int64_t kListedTets = 1000000;
 
 int rm_launch_pack(const int32_t* indices, const float* vertices, const float* cell, int64_t T, int64_t V,
@@ -2056,8 +2055,8 @@ int rm_launch_backward_finish(const int32_t* indices, const float* vertices, con
   if (t_end <= t_begin) return RM_OK;
   RmProfScope prof("k_backward_finish", st);
   const int64_t n = t_end - t_begin;
-  const int per = n > kListedTets ? 4 : 1;
-  auto kernel = per == 4 ? rm::k_backward_finish<4> : rm::k_backward_finish<1>;
+  const int per = n > kListedTets ? 3 : 1;
+  auto kernel = per == 3 ? rm::k_backward_finish<3> : rm::k_backward_finish<1>;
   const int64_t per_block = (int64_t)per * rm::kFinishThreads;
   RM_CUDA_CHECK(rm_launch(kernel, (unsigned)((n + per_block - 1) / per_block), rm::kFinishThreads, 0, st, indices, vertices, cell,
                           t_begin, t_end, *cam, reinterpret_cast<const float4*>(grec), hits->tet_flags, vgrad, cgrad));
