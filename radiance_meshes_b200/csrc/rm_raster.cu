@@ -1274,7 +1274,7 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
 constexpr int kBwdBatch = 8;          // entries per half-warp and round
 constexpr int kBwdStageStride = 7;    // float4 per staged record (6 used), as in the forward kernel
 
-struct BwdShared {                                // 11.1 KB: five blocks of four warps per SM
+struct BwdShared {                                // 11.1 KB: five blocks of four warps per SM, 19 of one warp (a block takes 1 KB more)
   float4 stage[2 * kBwdBatch * kBwdStageStride];  // refilled while phase B runs
   float4 planes[2 * kBwdBatch * 16];              // [slot]: (uq, q) of the entering and the leaving plane
   float4 fields[2 * kBwdBatch * 16];              // a, w, b, planes as one bit each (entering 2 i, leaving 2 i + 1)
@@ -1285,12 +1285,12 @@ struct BwdShared {                                // 11.1 KB: five blocks of fou
 // first; what the two entries change of the state is handed over by shuffles.  Both phases then take half as many rounds in
 // a row (13k tets, 128 x 128: 70 -> 49 us; 60k, 203 x 317: 154 -> 123 us; 2M, 300 x 300: 543 -> 459 us).
 // On its small grids a block of one warp: units of uneven length then do not hold each other's places (13k tets, 128 x 128:
-// 51.6 us with four, 47.6 with one; 2M of a scene, 300 x 300: 440 and 365).  Large grids lose by it what neighbouring units
-// share (6M: 2202 us with four, 2245 with one).
+// 49.3 us with four, 45.4 with one; 2M of a scene, 300 x 300: 451 and 445, 430 x 430: 717 and 715; 60k, 203 x 317: the same).
+// Large grids lose by it what neighbouring units share (6M: 2202 us with four, 2245 with one).
 template <bool PAIR>
 constexpr int kBwdWarps = PAIR ? 1 : kWarpsPerBlock;
 template <bool PAIR>
-__global__ void __launch_bounds__(kBwdWarps<PAIR> * 32, 20 / kBwdWarps<PAIR>)
+__global__ void __launch_bounds__(kBwdWarps<PAIR> * 32, PAIR ? 19 : 5)
 k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
            const float2* __restrict__ jitter, const float4* __restrict__ out_img, const float* __restrict__ dist_img,
            const int32_t* __restrict__ hit_counts, const int32_t* __restrict__ hit_ids,
