@@ -1,5 +1,6 @@
-"""Meshes of more than a million tets, where packing and the chain rule work through lists of the tets that need it, against
-the same tets in a small mesh, where a thread takes every tet."""
+"""Meshes of more than a million tets, where packing works through lists of the tets that need a record, against the same tets in
+a small mesh, where a thread packs every tet.  (The chain rule lists its tets in either; test_gpu_chain_rule.py has it against
+64 bits.)"""
 import numpy as np
 import pytest
 import torch
