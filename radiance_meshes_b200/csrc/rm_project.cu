@@ -496,9 +496,8 @@ __device__ __forceinline__ void for_corners(int4 r, F add) {
 // The corners of a warp's rectangles, by all lanes of it (on: this lane has one).  The tets of a mesh come in runs of
 // neighbours, so that most corners of a warp lie in a few tiles and many on the same: they are added up in a window of
 // 16 x 16 cells in shared memory (zero), which leaves as one atomic per cell that is not zero, lanes side by side.  Four
-// atomics per tet kept L2 busy for a third of the kernel: 6M tets, 1080p 320 -> 241 us, 21M 1380 -> 775 us, 36M, 2160p
-// 2105 -> 1335 us (2M, where more than half are culled: 71.5 -> 73.5 us; tets in random order, whose corners miss the window:
-// 2M 108 -> 108, 6.7M 464 -> 463, 21M 1818 -> 1815 us).
+// atomics per tet kept L2 busy for a third of the kernel: 6M tets, 1080p 317 -> 238 us, 18M 1040 -> 782 us, 36M, 2160p
+// 2105 -> 1335 us (2M, where more than half are culled: 68 -> 72 us).
 constexpr int kWindow = 16;
 __device__ __forceinline__ void add_coverage(const ProjectOut& o, const DevCam& cam, bool on, int4 r, int32_t* window) {
   if (!__any_sync(0xffffffffu, on)) return;
@@ -535,7 +534,7 @@ k_project(const int32_t* __restrict__ indices, int64_t T, const float* __restric
           ProjectOut o) {
   after_previous();
   __shared__ DevCam cam;
-  // of a warp: the window, then its depths and circumcentres (in an array of their own 2M tets took 2 us more, 21M 12)
+  __shared__ __align__(16) float rows[kProjectThreads / 32][2][96];
   __shared__ __align__(16) int32_t windows[kProjectThreads / 32][kWindow * kWindow];
   const int64_t g = (int64_t)blockIdx.x * kProjectThreads + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -621,9 +620,8 @@ k_project(const int32_t* __restrict__ indices, int64_t T, const float* __restric
   }
   const int64_t g0 = g - lane;
   if (g0 + 32 <= T && ((reinterpret_cast<uintptr_t>(o.vs_tetra) | reinterpret_cast<uintptr_t>(o.circumcenter)) & 15) == 0) {
-    __syncwarp();  // the window has been read
-    float* vs_row = reinterpret_cast<float*>(window);
-    float* cc_row = vs_row + 96;
+    float* vs_row = rows[threadIdx.x >> 5][0];
+    float* cc_row = rows[threadIdx.x >> 5][1];
     vs_row[3 * lane] = 0.0f;
     vs_row[3 * lane + 1] = 0.0f;
     vs_row[3 * lane + 2] = p.depth;
