@@ -496,8 +496,9 @@ __device__ __forceinline__ void for_corners(int4 r, F add) {
 // The corners of a warp's rectangles, by all lanes of it (on: this lane has one).  The tets of a mesh come in runs of
 // neighbours, so that most corners of a warp lie in a few tiles and many on the same: they are added up in a window of
 // 16 x 16 cells in shared memory (zero), which leaves as one atomic per cell that is not zero, lanes side by side.  Four
-// atomics per tet kept L2 busy for a third of the kernel: 6M tets, 1080p 317 -> 238 us, 18M 1040 -> 782 us, 36M, 2160p
-// 2105 -> 1335 us (2M, where more than half are culled: 68 -> 72 us).
+// atomics per tet kept L2 busy for a third of the kernel: 6M tets, 1080p 320 -> 241 us, 21M 1380 -> 785 us, 36M, 2160p
+// 2250 -> 1334 us; 2M, where more than half are culled: 70 -> 74 us, and half of a scene of 0.6M 30 -> 32.  In random order the
+// corners miss the window: 2M 106.5 -> 109 us, 6.7M 464 -> 465, 21M 1827 -> 1829.
 constexpr int kWindow = 16;
 __device__ __forceinline__ void add_coverage(const ProjectOut& o, const DevCam& cam, bool on, int4 r, int32_t* window) {
   if (!__any_sync(0xffffffffu, on)) return;
