@@ -1263,33 +1263,60 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
 //        to its entering and its leaving plane   (uq d, q)     with q = -dL/dt / den, u = distance from the camera
 //        to the colour gradient and its offset   (a d, w G)    with G = g.r + g.g + g.b
 //        to the base colour and the density      (w g, b)
-//      so seven floats and the two plane numbers leave for shared memory, 32 bytes, in place of 16 values.
+//      so seven floats leave for shared memory, and the two plane numbers as one byte.
 //   B. lane = (entry, half of its row).  The lane adds up its half of the entry's 24 record gradients over the 16
 //      pixels, in registers, reading each hit's scalars and the pixel's constants, and adds the sums to the row
 //      in global memory with 128-bit reductions: one per plane that the entry has hits on, two for the colours.
 // Lanes of phase A are on different entries at the same time, so none waits for entries that its pixel missed, and
-// phase B needs no shuffles, no ballots and no test of which pixels share faces.  Issue slots bound the kernel.
-// 1.98M tets, 822 x 1237, camera inside: 4.1e9 warp instructions in 4.88 ms for a lock-step walk over the entries
-// with a reduction per step, 2.2e9 in 2.58 ms for this; 6M tets, 1080p: 3.82 -> 1.94 ms.
+// phase B needs no shuffles and no test of which pixels share faces.  Issue slots bound the kernel, so what phase B does per
+// pixel is cut to loads, tests and additions:
+//   * A ray in front of the near plane enters through planes that face the camera and leaves through the others, which the
+//     sign of a plane's D tells.  A lane therefore loads the pair of its plane (8 bytes) and no other, and one bit of the
+//     pixel's byte says whether it counts: a predicate on the multiply-adds, where a selection between both pairs and zero
+//     takes eight instructions a pixel.
+// A near plane behind the camera (BEHIND) has rays that enter and leave on the same side of it: there phase B looks at both pairs.
+// (u = -D / den, so q u = dL/dt u^2 / D, and without the reciprocals, whose pick by plane costs six instructions a hit, 2M tets
+// would take 2.33 ms; but the sums, divided by D at the end, are 3 % further from 64 bits.)
+// With selections in phase B and 8 ballots a round for who has hit what: 2M tets, 822 x 1237,
+// 2.70 ms, 6.7M, 1080p, 2.14, 21M 3.61, a medium scene 1.04e9 warp instructions; now 2.43, 1.92, 3.07 ms, 0.9e9.  (A lock-step walk
+// over the entries with a reduction per step took twice that.)
 constexpr int kBwdBatch = 8;          // entries per half-warp and round
 constexpr int kBwdStageStride = 7;    // float4 per staged record (6 used), as in the forward kernel
 
-struct BwdShared {                                // 11.1 KB: five blocks of four warps per SM, 19 of one warp (a block takes 1 KB more)
-  float4 stage[2 * kBwdBatch * kBwdStageStride];  // refilled while phase B runs
-  float4 planes[2 * kBwdBatch * 16];              // [slot]: (uq, q) of the entering and the leaving plane
-  float4 fields[2 * kBwdBatch * 16];              // a, w, b, planes as one bit each (entering 2 i, leaving 2 i + 1)
-  float4 pixel[16][2][2];                         // [pixel][half][0: d, G; 1: g, 1]
-  int id[2][2 * kBwdBatch];                       // [round & 1]
+// What phase A leaves of an entry: [pixel] (uq, q) of the entering and of the leaving plane, and (a, b, w, w).  The odd stride
+// in units of 16 bytes spreads the entries over the banks.
+struct BwdRow {
+  float4 planes[16], fields[16], unused;
 };
+struct BwdShared {                              // 11 KB: five blocks of four warps per SM, 19 of one warp (a block takes 1 KB more)
+  float4 stage[2 * kBwdBatch * kBwdStageStride];  // refilled while phase B runs; behind an entry's record, its 16 face bytes
+  BwdRow rows[2 * kBwdBatch];
+  float4 pixel[16][2][2];                         // [pixel][half][0: d, 1; 1: g, G]
+};
+constexpr int kFacesAt = 6;  // of an entry's staged record, in float4: a byte per pixel, entering plane 1 << 2 i, leaving 2 << 2 i
+
+// s + v (x, y, z1) where the word has one of the bits, v.x for the first three components and v.y for the last, whose constant
+// of the pixel is z1.y.
+__device__ __forceinline__ void add_where(unsigned word, unsigned bits, float2 v, float x, float y, float2 z1, float& sx, float& sy,
+                                          float2& sz) {
+  asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+      "and.b32 t, %3, %4;\n\tsetp.ne.u32 p, t, 0;\n\t"
+      "@p fma.rn.f32 %0, %5, %6, %0;\n\t"
+      "@p fma.rn.f32 %1, %5, %7, %1;\n\t"
+      "@p fma.rn.f32x2 %2, %8, %9, %2;\n\t}"
+      : "+f"(sx), "+f"(sy), "+l"(reinterpret_cast<unsigned long long&>(sz))
+      : "r"(word), "r"(bits), "f"(v.x), "f"(x), "f"(y), "l"(reinterpret_cast<unsigned long long&>(v)),
+        "l"(reinterpret_cast<unsigned long long&>(z1)));
+}
 // PAIR: one unit per warp, 16 entries a round and two lanes per pixel, each on every other entry of the pixel, the last
 // first; what the two entries change of the state is handed over by shuffles.  Both phases then take half as many rounds in
 // a row (13k tets, 128 x 128: 70 -> 49 us; 60k, 203 x 317: 154 -> 123 us; 2M, 300 x 300: 543 -> 459 us).
-// On its small grids a block of one warp: units of uneven length then do not hold each other's places (13k tets, 128 x 128:
-// 49.3 us with four, 45.4 with one; 2M of a scene, 300 x 300: 451 and 445, 430 x 430: 717 and 715; 60k, 203 x 317: the same).
+// On its small grids a block of one warp: units of uneven length then do not hold each other's places (with selections in phase B,
+// 13k tets, 128 x 128: 49.3 us with four, 45.4 with one; 2M of a scene, 300 x 300: 451 and 445, 430 x 430: 717 and 715; 60k, 203 x 317: the same).
 // Large grids lose by it what neighbouring units share (6M: 2202 us with four, 2245 with one).
 template <bool PAIR>
 constexpr int kBwdWarps = PAIR ? 1 : kWarpsPerBlock;
-template <bool PAIR>
+template <bool PAIR, bool BEHIND>
 __global__ void __launch_bounds__(kBwdWarps<PAIR> * 32, PAIR ? 19 : 5)
 k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
            const float2* __restrict__ jitter, const float4* __restrict__ out_img, const float* __restrict__ dist_img,
@@ -1305,7 +1332,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   const bool second = PAIR && lane >= 16;
   BwdShared& sm = reinterpret_cast<BwdShared*>(smem_bwd)[warp];
   float4* const staged = sm.stage + half * kBwdBatch * kBwdStageStride;
-  float4 *const planes = sm.planes + half * kBwdBatch * 16, *const fields = sm.fields + half * kBwdBatch * 16;
+  BwdRow* const rows = sm.rows + half * kBwdBatch;
   const int64_t unit = ((int64_t)blockIdx.x * kBwdWarps<PAIR> + warp) * (PAIR ? 1 : 2) + half;
   Unit u = make_unit(rcam, ranges, unit, n_units, subs, lane16);
 
@@ -1326,8 +1353,8 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
     gv = __ldg(gd + 4) * (1.0f / 3.0f);
   }
   const float G = gr + gg + gb;
-  sm.pixel[lane16][half][0] = make_float4(d.x, d.y, d.z, G);
-  sm.pixel[lane16][half][1] = make_float4(gr, gg, gb, 1.0f);
+  sm.pixel[lane16][half][0] = make_float4(d.x, d.y, d.z, 1.0f);
+  sm.pixel[lane16][half][1] = make_float4(gr, gg, gb, G);
   const float min_t = rcam.min_t;
 
   // The half-warp's hit list (written by the forward pass: the batches of 16 it evaluated, each with its tet ids
@@ -1360,7 +1387,6 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   };
   auto stage = [&](int k) {
     if (k < rounds) {
-      if (part == 0) sm.id[k & 1][half * kBwdBatch + ent] = id_next;
       const float4* src = records + record_at(id_next) + 3 * part;
       float4* dst = staged + ent * kBwdStageStride + 3 * part;
 #pragma unroll
@@ -1369,21 +1395,23 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
     cp_async_commit();
   };
   const Ray ray = make_ray(d);
+  // what phase A leaves of a hit: an entering distance te <= 0 is clamped and has no gradient
+  auto leave = [&](int j, const Crossing& cr, float te, float g_enter, float g_exit, float a, float b, float w) {
+    const float q_e = te > 0.0f ? -g_enter * cr.r_e : 0.0f, q_x = -g_exit * cr.r_x;
+    rows[j].planes[lane16] = make_float4(q_e * cr.ue, q_e, q_x * cr.ux, q_x);
+    rows[j].fields[lane16] = make_float4(a, b, w, w);
+    reinterpret_cast<uint8_t*>(staged + j * kBwdStageStride + kFacesAt)[lane16] = (uint8_t)cr.faces;
+  };
+  float4* const faces_row = staged + ent * kBwdStageStride + kFacesAt;
+  if (part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
   fetch(rounds - 1);
   stage(0);
   for (int k = 0; k < max_rounds; ++k) {
     unsigned bits = bits_next;
+    const int id = id_next;  // of the entry this lane sums
     fetch(rounds - 2 - k);
     cp_async_wait<0>();
     __syncwarp();
-    // pixels that hit the entry this lane sums
-    unsigned mine = 0;
-#pragma unroll
-    for (int e = 0; e < kEntries; ++e) {
-      const unsigned col = __ballot_sync(FULL, (bits >> e) & 1u);
-      if (ent == e) mine = col;
-    }
-    mine = (mine >> (16 * half)) & 0xFFFFu;
 
     // ---- phase A
     if constexpr (PAIR) {
@@ -1395,7 +1423,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
       while (__any_sync(FULL, bits != 0u)) {
         const int j = 31 - __clz(bits);  // -1 where no entry is left
         Crossing cr = {};
-        float4 cg = make_float4(0.f, 0.f, 0.f, 0.f), cb = cg, o_planes = cg, o_fields = cg;
+        float4 cg = make_float4(0.f, 0.f, 0.f, 0.f), cb = cg;
         if (j >= 0) {
           bits ^= 1u << j;
           const float4* rec = staged + j * kBwdStageStride;
@@ -1434,13 +1462,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
           const float b = fmaf(fmaf(2.0f, gvd, g_tau), dt, fmaf(g_m1, mid, g_m0));
           const float g_dt = fmaf(gvd, dens, g_tau * dens), g_mid = 0.5f * g_m1 * dens;
           const float g_exit = fmaf(g_ox, gd, g_mid) + g_dt, g_enter = fmaf(g_oe, gd, g_mid) - g_dt;
-          const float q_e = te > 0.0f ? -g_enter * cr.r_e : 0.0f, q_x = -g_exit * cr.r_x;
-          o_planes = make_float4(q_e * cr.ue, q_e, q_x * cr.ux, q_x);
-          o_fields = make_float4(fmaf(g_ox, X, g_oe * E), w * Tp, b, __uint_as_float(cr.faces));
-        }
-        if (j >= 0) {
-          planes[entry_slot(j, lane16)] = o_planes;
-          fields[entry_slot(j, lane16)] = o_fields;
+          leave(j, cr, te, g_enter, g_exit, fmaf(g_ox, X, g_oe * E), b, w * Tp);
         }
         logT = logT2;
         sz = sz2;
@@ -1456,7 +1478,6 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
       const float4* rec = staged + j * kBwdStageStride;
       const float4 pl[4] = {rec[0], rec[1], rec[2], rec[3]};
       const float4 cg = rec[4], cb = rec[5];
-      float4 o_planes = make_float4(0.f, 0.f, 0.f, 0.f), o_fields = o_planes;
       const Crossing cr = slab_planes(pl, ray);
       // A hit has entered before it leaves and leaves in front of the origin, so the leaving distance needs no
       // clamp.  (The forward pass found the optical depth positive with the same operations; the test only keeps
@@ -1494,39 +1515,57 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
         const float g_dt = fmaf(gvd, dens, g_tau * dens), g_mid = 0.5f * g_m1 * dens;
         const float g_exit = fmaf(g_ox, gd, g_mid) + g_dt, g_enter = fmaf(g_oe, gd, g_mid) - g_dt;
         // planes: t = u - min_t, u = -D/den  =>  dt/dD = -1/den, dt/dn = -u/den d
-        const float q_e = te > 0.0f ? -g_enter * cr.r_e : 0.0f, q_x = -g_exit * cr.r_x;
-        o_planes = make_float4(q_e * cr.ue, q_e, q_x * cr.ux, q_x);
-        o_fields = make_float4(fmaf(g_ox, X, g_oe * E), w * Tp, b, __uint_as_float(cr.faces));
+        leave(j, cr, te, g_enter, g_exit, fmaf(g_ox, X, g_oe * E), b, w * Tp);
       }
-      planes[entry_slot(j, lane16)] = o_planes;
-      fields[entry_slot(j, lane16)] = o_fields;
     }
     __syncwarp();
+    // the entry's face bytes and the signs of its two planes' -D, before the copies of the next round and its phase A write there
+    const float4 f4 = *faces_row;
+    const float2 neg_d = reinterpret_cast<const float2*>(staged + ent * kBwdStageStride + 2 * part + 1)[1];
+    const unsigned faces[4] = {__float_as_uint(f4.x), __float_as_uint(f4.y), __float_as_uint(f4.z), __float_as_uint(f4.w)};
+    __syncwarp();
+    if (part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
     stage(k + 1);
 
-    // ---- phase B: part 0 sums planes 0 and 1 and the colour gradient, part 1 planes 2 and 3 and base colour, density
-    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0, sf = s0;
-#pragma unroll 4
+    // ---- phase B: part 0 sums planes 0 and 1, the colour gradient and the density, part 1 planes 2 and 3, the base colour and
+    // the offset of the colour gradient; x, y and (z, the row's last)
+    const BwdRow& row = rows[ent];
+    const float2* const plane_pairs = reinterpret_cast<const float2*>(row.planes);
+    const float2* const field_pairs = reinterpret_cast<const float2*>(row.fields) + part;
+    int side0 = neg_d.x < 0.0f ? 0 : 1, side1 = neg_d.y < 0.0f ? 0 : 1;  // entering (facing the camera) or leaving
+    float x0 = 0.f, y0 = 0.f, x1 = 0.f, y1 = 0.f, xf = 0.f, yf = 0.f;
+    float2 z0 = {0.f, 0.f}, z1 = z0, zf = z0;
+    const unsigned plane0 = 0x01010101u << (4 * part), plane1 = 0x04040404u << (4 * part);
+    unsigned bits0 = plane0 << side0, bits1 = plane1 << side1;
+#pragma unroll
     for (int p = 0; p < 16; ++p) {
-      const bool has = (mine >> p) & 1u;  // else the slot holds nothing of this round
-      const float4 pq = planes[entry_slot(ent, p)], f = fields[entry_slot(ent, p)];
+      const unsigned byte = 0xFFu << (8 * (p & 3));
       const float4 dir = sm.pixel[p][half][0], con = sm.pixel[p][half][part];
-      const unsigned faces = has ? __float_as_uint(f.w) >> (4 * part) : 0u;
-      const float u0 = faces & 1u ? pq.x : (faces & 2u ? pq.z : 0.0f), q0 = faces & 1u ? pq.y : (faces & 2u ? pq.w : 0.0f);
-      const float u1 = faces & 4u ? pq.x : (faces & 8u ? pq.z : 0.0f), q1 = faces & 4u ? pq.y : (faces & 8u ? pq.w : 0.0f);
-      s0.x = fmaf(u0, dir.x, s0.x); s0.y = fmaf(u0, dir.y, s0.y); s0.z = fmaf(u0, dir.z, s0.z); s0.w += q0;
-      s1.x = fmaf(u1, dir.x, s1.x); s1.y = fmaf(u1, dir.y, s1.y); s1.z = fmaf(u1, dir.z, s1.z); s1.w += q1;
-      const float fa = has ? (part ? f.y : f.x) : 0.0f, fb = has ? (part ? f.z : f.y) : 0.0f;
-      sf.x = fmaf(fa, con.x, sf.x); sf.y = fmaf(fa, con.y, sf.y); sf.z = fmaf(fa, con.z, sf.z);
-      sf.w = fmaf(fb, con.w, sf.w);
+      add_where(faces[p >> 2], bits0 & byte, plane_pairs[2 * p + side0], dir.x, dir.y, {dir.z, dir.w}, x0, y0, z0);
+      add_where(faces[p >> 2], bits1 & byte, plane_pairs[2 * p + side1], dir.x, dir.y, {dir.z, dir.w}, x1, y1, z1);
+      add_where(faces[p >> 2], byte, field_pairs[2 * p], con.x, con.y, {con.z, con.w}, xf, yf, zf);
     }
-    if (mine) {
-      float4* row = reinterpret_cast<float4*>(grec + (int64_t)sm.id[k & 1][half * kBwdBatch + ent] * 24);
-      if (s0.x != 0.f || s0.y != 0.f || s0.z != 0.f || s0.w != 0.f) atomicAdd(row + 2 * part, s0);
-      if (s1.x != 0.f || s1.y != 0.f || s1.z != 0.f || s1.w != 0.f) atomicAdd(row + 2 * part + 1, s1);
-      atomicAdd(row + 4 + part, sf);
+    if constexpr (BEHIND) {  // the pairs of the other side
+      side0 ^= 1;
+      side1 ^= 1;
+#pragma unroll 1
+      for (int p = 0; p < 16; ++p) {
+        const unsigned byte = 0xFFu << (8 * (p & 3)), word = reinterpret_cast<const unsigned*>(&f4)[p >> 2];
+        const float4 dir = sm.pixel[p][half][0];
+        add_where(word, (plane0 << side0) & byte, plane_pairs[2 * p + side0], dir.x, dir.y, {dir.z, dir.w}, x0, y0, z0);
+        add_where(word, (plane1 << side1) & byte, plane_pairs[2 * p + side1], dir.x, dir.y, {dir.z, dir.w}, x1, y1, z1);
+      }
+      bits0 = plane0 * 3u;
+      bits1 = plane1 * 3u;
     }
-    __syncwarp();
+    const unsigned any = faces[0] | faces[1] | faces[2] | faces[3];
+    const float last = __shfl_xor_sync(FULL, zf.y, 1);  // the density's sum belongs to the row of part 1, the offset's to part 0's
+    if (any) {
+      float4* out = reinterpret_cast<float4*>(grec + (int64_t)id * 24);
+      if (any & bits0) atomicAdd(out + 2 * part, make_float4(x0, y0, z0.x, z0.y));
+      if (any & bits1) atomicAdd(out + 2 * part + 1, make_float4(x1, y1, z1.x, z1.y));
+      atomicAdd(out + 4 + part, make_float4(xf, yf, zf.x, last));
+    }
   }
   cp_async_wait<0>();
 }
@@ -2017,7 +2056,9 @@ static int launch_backward_walk(const int32_t* ranges, const float* records, con
   const int warps = pair ? rm::kBwdWarps<true> : rm::kBwdWarps<false>;
   if (pair) blocks = (unsigned)((n_units + warps - 1) / warps);
   const size_t smem = warps * sizeof(rm::BwdShared);
-  auto kernel = pair ? rm::k_backward<true> : rm::k_backward<false>;
+  const bool behind = !(cam->min_t >= 0.0f);
+  auto kernel = pair ? (behind ? rm::k_backward<true, true> : rm::k_backward<true, false>)
+                     : (behind ? rm::k_backward<false, true> : rm::k_backward<false, false>);
   RM_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   RmProfScope prof("k_backward", st);
   RM_CUDA_CHECK(rm_launch_behind(T, kernel, blocks, warps * 32, smem, st,
