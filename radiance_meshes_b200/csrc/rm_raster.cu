@@ -74,11 +74,18 @@ __device__ __forceinline__ float pack_normal(float x, float y) {  // each with a
   return __uint_as_float((unsigned)(__float2int_rn(x * kLineUnit) + 32768) |
                          (unsigned)(__float2int_rn(y * kLineUnit) + 32768) << 16);
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
 __device__ __forceinline__ float2 unpack_normal(float f) {
   // 2^23 + u is a float whose low mantissa bits are u
   const unsigned u = __float_as_uint(f);
-  return make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7410)) - 8421376.0f,
-                     __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7432)) - 8421376.0f);
+  return add2(make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7432))),
+              make_float2(-8421376.0f, -8421376.0f));
 }
 __device__ __forceinline__ HullLines unpack_lines(float4 l0, float4 l1) {
   const float2 p0 = unpack_normal(l0.x), p1 = unpack_normal(l0.z), p2 = unpack_normal(l1.x), p3 = unpack_normal(l1.z);
@@ -309,8 +316,9 @@ k_pack_records(const int32_t* __restrict__ indices, const float* __restrict__ ve
 }
 
 // Box of the samples of a half-warp: centre, half extents, and how far outside a line it counts as missed.
-struct alignas(16) SampleBox {
-  float x, y, ex, ey, margin, unused[3];
+struct SampleBox {
+  float4 box;  // x, y, half extents
+  float margin;
 };
 // True if one of the four hull lines of a tet has the whole box on its outer side by more than the margin.
 // Conservative: NaN lines never separate.
@@ -319,7 +327,7 @@ __device__ __forceinline__ bool hull_misses_box(float4 l0, float4 l1, const Samp
   float v[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k)  // largest value of the line over the box
-    v[k] = fmaf(fabsf(h.a[k]), s.ex, fmaf(fabsf(h.b[k]), s.ey, fmaf(h.a[k], s.x, fmaf(h.b[k], s.y, h.c[k]))));
+    v[k] = fmaf(fabsf(h.a[k]), s.box.z, fmaf(fabsf(h.b[k]), s.box.w, fmaf(h.a[k], s.box.x, fmaf(h.b[k], s.box.y, h.c[k]))));
   return fminf(fminf(v[0], v[1]), fminf(v[2], v[3])) < -s.margin;
 }
 
@@ -424,13 +432,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   float2 r;
   asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long&>(r))
-      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
-  return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("add.rn.f32x2 %0, %1, %2;"
       : "=l"(reinterpret_cast<unsigned long long&>(r))
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
   return r;
@@ -560,6 +561,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -625,8 +630,8 @@ __device__ __forceinline__ SampleBox halfwarp_sample_box(bool inside, float2 s, 
     y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
     y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
   }
-  if (lost & 0xFFFFu) return {0.f, 0.f, 0.f, 0.f, 3.0e38f, {}};  // only a tet that no ray can hit misses it
-  return {0.5f * (x0 + x1), 0.5f * (y0 + y1), 0.5f * (x1 - x0), 0.5f * (y1 - y0), margin, {}};
+  if (lost & 0xFFFFu) return {{0.f, 0.f, 0.f, 0.f}, 3.0e38f};  // only a tet that no ray can hit misses it
+  return {{0.5f * (x0 + x1), 0.5f * (y0 + y1), 0.5f * (x1 - x0), 0.5f * (y1 - y0)}, margin};
 }
 
 // ----------------------------------------------------------------------------
@@ -634,10 +639,11 @@ __device__ __forceinline__ SampleBox halfwarp_sample_box(bool inside, float2 s, 
 // ----------------------------------------------------------------------------
 // A half-warp owns 16 pixels of one tile and walks the tile's list in three stages that
 // are decoupled by two small queues in shared memory (ring buffers of 32 slots):
-//   1. examination, 16 entries at a time: every lane reads the hull lines of one entry
-//      (32 bytes, on their way to shared memory two steps ahead) and tests them against the
-//      bounding box of the half-warp's samples (k_pack_records marks the lines of a tet of
-//      zero density); survivors go to queue A in list order with their position;
+//   1. examination, 16 entries at a time: every lane tests the hull lines of one entry
+//      (32 bytes, on their way to shared memory three steps ahead, their tet ids as many
+//      before that) against the bounding box of the half-warp's samples (k_pack_records marks
+//      the lines of a tet of zero density); survivors go to queue A in list order with their
+//      position and their lines;
 //   2. when both half-warps hold 16 entries in queue A (or have nothing left to examine),
 //      every lane takes one of them and tests the hull lines against each of the 16 sample
 //      positions, which gives the mask of the pixels whose ray can touch the tet; entries
@@ -655,23 +661,36 @@ __device__ __forceinline__ SampleBox halfwarp_sample_box(bool inside, float2 s, 
 // the tet ids of the batch and, per pixel, the bit set of the batch entries it hit.
 constexpr int kBatch = 16;       // entries staged and evaluated per half-warp and round
 constexpr int kRing = 32;        // slots of each candidate queue
-constexpr int kStageStride = 7;  // float4 per staged record: 6 used; the odd stride spreads the records over the banks
+// Examination steps whose hull lines are on their way; tet ids are read as many steps before that.  A step is 100 instructions and
+// waited 1,360 cycles for its ids and lines, as did stage 2 for its lines, when these were read one step ahead and from L1: 2M tets,
+// 822 x 1237, 2.01 ms, 6.7M, 1080p, 1.83, 36M, 2160p, 7.39, constant colour, 600k, 800 x 800, 0.54; now 1.78, 1.63, 6.67, 0.52, of
+// which the order of a step (copies before the test) is 2 %.  Before, 59 % of the issue slots; now 70 %, with 4 % more instructions.
+constexpr int kAhead = 3;
 
+// An examination step on its way: hull lines of its entries, first and second 16 bytes apart by a distance at which two lanes
+// that copy the two of one entry meet no bank twice, and tet ids, of this step and of the one kAhead later in turn.
+struct ExamStep {
+  float4 low[32], gap[4], high[32];
+  int ids[2][32];
+};
 // What a warp keeps in shared memory.  What the evaluation loop does not need - hull lines on their way to the
-// examination, sample box, hit-list positions - lives here and not in registers.  Five blocks of four warps per SM:
-// six (80 registers) fill no more issue slots, because the loads of the evaluation loop then take the shared-memory
-// pipe to 64 % (6M tets, 1080p: 1.98 ms with five, 2.28 ms with six).
-struct FwdShared {
-  float4 stage[2 * kBatch * kStageStride];
-  float4 lines[2][32 * 2];                 // [buffer][lane]: hull lines of the entries examined next
+// examination, sample box, hit-list positions - lives here and not in registers.  11.4 KB: five blocks of four warps per SM.
+template <int STRIDE>
+struct WalkShared {
+  float4 stage[2 * kBatch * STRIDE];
+  ExamStep steps[kAhead];                  // [step % kAhead]; the gap of the first two: what `box` and `hits` return
+  float4 a_low[2 * kRing], a_high[2 * kRing];  // hull lines of the entries in queue A
   float4 samples[8][2];                    // [pair][half]: two samples each: x0, x1, y0, y1
-  SampleBox box[2];                        // [half]
-  int64_t hits[2][2];                      // [half]: first id slot and first mask slot of the hit list
+  uint16_t batch_mask[2 * kBatch];         // entries e and e + 8 of 16 in one word
   int a_id[2 * kRing], a_pos[2 * kRing];
   int b_id[2 * kRing], b_pos[2 * kRing];
-  uint32_t b_mask[2 * kRing];
+  uint16_t b_mask[2 * kRing];
   int batch_id[2 * kBatch], batch_pos[2 * kBatch];
-  uint32_t batch_mask[2 * kBatch];
+
+  __device__ __forceinline__ float4* box(int half) { return &steps[0].gap[2 * half]; }  // centre and half extents, then the margin
+  __device__ __forceinline__ int64_t* hits(int half) {  // first id slot and first mask slot of the hit list
+    return reinterpret_cast<int64_t*>(&steps[1].gap[half]);
+  }
 };
 
 // The Tukey power ladder of the constant-colour variant (slang/alphablend_shader.slang:26-33):
@@ -706,18 +725,18 @@ __device__ __forceinline__ uint32_t hull_sample_mask(float4 l0, float4 l1, const
   return ~outside & 0xFFFFu;
 }
 
-// Bit j of the result = bit `lane16` of word j of the 16 masks at `masks` (16-byte aligned).
-__device__ __forceinline__ uint32_t transpose_masks(const uint32_t* __restrict__ masks, int lane16) {
+// Bit j of the result = bit `lane16` of the mask of entry j of 16; word i (of 8, 16-byte aligned) holds entries i and i + 8.
+__device__ __forceinline__ uint32_t transpose_masks(const uint16_t* __restrict__ masks, int lane16) {
   uint32_t bits = 0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 2; ++q) {
     const uint4 w = reinterpret_cast<const uint4*>(masks)[q];
-    bits |= ((w.x >> lane16) & 1u) << (4 * q);
-    bits |= ((w.y >> lane16) & 1u) << (4 * q + 1);
-    bits |= ((w.z >> lane16) & 1u) << (4 * q + 2);
-    bits |= ((w.w >> lane16) & 1u) << (4 * q + 3);
+    bits |= ((w.x >> lane16) & 0x10001u) << (4 * q);
+    bits |= ((w.y >> lane16) & 0x10001u) << (4 * q + 1);
+    bits |= ((w.z >> lane16) & 0x10001u) << (4 * q + 2);
+    bits |= ((w.w >> lane16) & 0x10001u) << (4 * q + 3);
   }
-  return bits;
+  return (bits & 0xFFu) | (bits >> 8);
 }
 
 // MODE kColor: the interpolated-colour renderer (slang/alphablend_shader_interp.slang).
@@ -740,7 +759,11 @@ __device__ __forceinline__ uint32_t transpose_masks(const uint32_t* __restrict__
 enum ForwardMode { kColor, kConstColor, kStats };
 constexpr int kStatsBatch = 8;  // entries whose hits are in shared memory at a time
 
-struct StatsShared : FwdShared {
+// float4 per staged record: 6 used, of the statistics, which need no colours, 5; the odd stride spreads the records over the banks
+template <ForwardMode MODE>
+constexpr int kStageStride = MODE == kStats ? 5 : 7;
+using FwdShared = WalkShared<kStageStride<kColor>>;
+struct StatsShared : WalkShared<kStageStride<kStats>> {
   float4 hit[2 * kStatsBatch * 16 + 1];  // [half, entry_slot]: T, T * entry distance, T * exit distance; the last one: zeros
   float4 pixel[3][4][2][2];              // [component][four pixels][0: err, err^2, ssim; 1: ray direction][half]
 };
@@ -815,10 +838,12 @@ __device__ __forceinline__ void walk_unit(
   };
   int *const a_id = sm.a_id + half * kRing, *const a_pos = sm.a_pos + half * kRing;
   int *const b_id = sm.b_id + half * kRing, *const b_pos = sm.b_pos + half * kRing;
-  uint32_t* const b_mask = sm.b_mask + half * kRing;
+  float4 *const a_low = sm.a_low + half * kRing, *const a_high = sm.a_high + half * kRing;
+  uint16_t* const b_mask = sm.b_mask + half * kRing;
   int *const batch_id = sm.batch_id + half * kBatch, *const batch_pos = sm.batch_pos + half * kBatch;
-  uint32_t* const batch_mask = sm.batch_mask + half * kBatch;
-  float4* const stage = sm.stage + half * kBatch * kStageStride;
+  uint16_t* const batch_mask = sm.batch_mask + half * kBatch;
+  constexpr int kStride = kStageStride<MODE>;
+  float4* const stage = sm.stage + half * kBatch * kStride;
   Unit u = make_unit(rcam, ranges, unit, n_units, subs, lane16);
   if (u.len > skip_length) {
     u.inside = false;
@@ -837,12 +862,13 @@ __device__ __forceinline__ void walk_unit(
     sp[2] = sample.y;
     const SampleBox box = halfwarp_sample_box(u.inside, sample, rcam.camera_type == 1 ? kFisheyeMargin : kPixelMargin);
     if (lane16 == 0) {
-      sm.box[half] = box;
+      sm.box(half)[0] = box.box;
+      sm.box(half)[1].x = box.margin;
       // Hit list of this half-warp: the tet ids of every evaluated batch at [first, first + n_ent), and for batch b
       // the 16 per-pixel bit sets behind the mask slot.  Every batch but the last holds 16 entries.
       const int64_t first = (int64_t)u.start * u.subs + (int64_t)u.sub * u.len;
-      sm.hits[half][0] = first;
-      sm.hits[half][1] = first + 16 * ((int64_t)u.tile * u.subs + u.sub);
+      sm.hits(half)[0] = first;
+      sm.hits(half)[1] = first + 16 * ((int64_t)u.tile * u.subs + u.sub);
     }
   }
   const Ray ray = make_ray(d);
@@ -871,32 +897,40 @@ __device__ __forceinline__ void walk_unit(
   bool fetching = act16 != 0;
   int n_ent = 0;  // entries in the hit list
 
-  // Examination: entry src + el is the one this lane examines next.  Its hull lines and those of the entry after it
-  // are in sm.lines or on their way (16-byte copies through L1, where stage 2 finds them again); of the entry after
-  // those the tet id is in flight.
+  // Examination: entry src + el is the one this lane examines next.  The hull lines of that step and of the two behind it are
+  // in sm.steps or on their way, and so are the tet ids of the three steps behind those.  All of it by asynchronous copies, two
+  // lanes for the lines of an entry, so that a sector is one access.  Behind the end of the list its last entry is copied.
   int src = 0;
   int qa_h = 0, qa_n = 0, qb_h = 0, qb_n = 0;  // ring heads and fill levels (the same in all lanes of the half)
-  auto list_id = [&](int e) {
-    int id = e < u.len ? __ldg(list + u.start + e) : -1;
-    if (id >= 0 && !RM_INDEX_OK(id, RM_X_TETS, 1)) id = -1;
-    return id;
-  };
-  auto fetch_lines = [&](int id, int buffer) {
-    if (id >= 0) {
-      const float4* rec = records + record_at(id) + kLinesAt;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) cp_async16_l1(&sm.lines[buffer][32 * k + lane], rec + k);
-    }
-    cp_async_commit();
-  };
   if (!fetching) u.len = 0;
-  int id_e = list_id(el), id_n = list_id(kEntries + el), id_n2 = list_id(2 * kEntries + el);
-  fetch_lines(id_e, 0);
-  fetch_lines(id_n, 1);
-  int buffer = 0;
+  const int last = u.len - 1;
+  const int32_t* const list_at = list + u.start;
+  const float4* const lines_at = records + kLinesAt + (el & 1);
+  ExamStep* step = sm.steps;
+  int turn = 0;  // which of the step's ids are its own
+  const int pair_lane = lane - el + (el >> 1);  // entry whose lines this lane copies, and the one kEntries / 2 on
+  auto fetch = [&](int first, ExamStep* st, int at) {  // lines of the step at `first` with the ids [at], ids of kAhead steps on
+    float4* const to = (el & 1 ? st->high : st->low) + pair_lane;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int id = st->ids[at][pair_lane + k * (kEntries / 2)];
+      if (RM_INDEX_OK(id, RM_X_TETS, 1)) cp_async16_l1(to + k * (kEntries / 2), lines_at + record_at(id));
+    }
+    cp_async4(&st->ids[at ^ 1][lane], list_at + min(first + kAhead * kEntries + el, last));
+  };
+  if (u.len > 0) {
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) sm.steps[k].ids[0][lane] = __ldg(list_at + min(k * kEntries + el, last));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) {
+    if (u.len > 0) fetch(k * kEntries, sm.steps + k, 0);
+    cp_async_commit();
+  }
 
   int n_cur = 0;   // entries of the staged batch
-  int since = 2;   // examination steps since records were staged, 2 for two or more
+  int since = kAhead;   // examination steps since records were staged
   __syncwarp();
   for (;;) {
     {
@@ -905,38 +939,41 @@ __device__ __forceinline__ void walk_unit(
     }
     // ---- stages 1 and 2: until both halves hold a full batch in queue B or have run dry
     for (;;) {
-      const bool need_b = fetching && qb_n < kEntries && (qa_n > 0 || src < u.len);
-      if (!__any_sync(FULL, need_b)) break;
-      const bool ready_a = !need_b || qa_n >= kEntries || src >= u.len;
-      if (!__all_sync(FULL, ready_a)) {
-        // Copies are committed by all lanes together: lines of this step, lines of the next, and, if records were staged
-        // within the last two steps, those behind the first or the second.
-        if (since < 2) cp_async_wait<2>(); else cp_async_wait<1>();
-        const bool examine = need_b && !ready_a;
-        bool cand = false;
-        if (examine && id_e >= 0) {
-          const float4* l = sm.lines[buffer] + lane;
-          cand = !hull_misses_box(l[0], l[32], sm.box[half]);
+      const bool hungry = fetching && qb_n < kEntries;
+      for (;;) {
+        const bool examine = hungry && qa_n < kEntries && src < u.len;
+        if (!__any_sync(FULL, examine)) break;
+        // Copies are committed by all lanes together.  Those of this step lie behind kAhead - 1 later ones; where records were
+        // staged since, their copies count as one of these, and a later step's are waited for, which began long before them.
+        cp_async_wait<kAhead - 1>();
+        __syncwarp();
+        const float4 l0 = step->low[lane], l1 = step->high[lane];
+        const int id = step->ids[turn][lane], pos = src + el;
+        __syncwarp();  // all lanes have read; the copies, which depend on nothing else, come before the long chain of the test
+        if (examine) {
+          fetch(src + kAhead * kEntries, step, turn ^ 1);
+          src += kEntries;
+          if (++step == sm.steps + kAhead) {
+            step = sm.steps;
+            turn ^= 1;
+          }
         }
+        cp_async_commit();
+        const bool cand = examine && pos <= last && !hull_misses_box(l0, l1, {sm.box(half)[0], sm.box(half)[1].x}) &&
+                          RM_INDEX_OK(id, RM_X_TETS, 1);
         const unsigned cb = unit_ballot(cand);
         if (cand) {
           const int slot = (qa_h + qa_n + __popc(cb & below)) & (kSlots - 1);
-          a_id[slot] = id_e;
-          a_pos[slot] = src + el;
+          a_id[slot] = id;
+          a_pos[slot] = pos;
+          a_low[slot] = l0;
+          a_high[slot] = l1;
         }
-        int id_fetch = -1;
-        if (examine) {
-          qa_n += __popc(cb);
-          src += kEntries;
-          id_e = id_n;
-          id_fetch = id_n = id_n2;
-          id_n2 = list_id(src + 2 * kEntries + el);
-        }
-        fetch_lines(id_fetch, buffer);
-        if (examine) buffer ^= 1;
-        since = min(since + 1, 2);
-        continue;
+        qa_n += __popc(cb);
+        ++since;
       }
+      const bool need_b = hungry && qa_n > 0;
+      if (!__any_sync(FULL, need_b)) break;
       __syncwarp();
       const int take_a = need_b ? min(qa_n, kEntries) : 0;
       uint32_t m = 0;
@@ -945,24 +982,24 @@ __device__ __forceinline__ void walk_unit(
         const int slot = (qa_h + el) & (kSlots - 1);
         cid = a_id[slot];
         cpos = a_pos[slot];
-        const float4* l = records + record_at(cid) + kLinesAt;
         const float margin = rcam.camera_type == 1 ? kFisheyeMargin : kPixelMargin;
-        m = hull_sample_mask(__ldg(l), __ldg(l + 1), sm.samples, half, margin) & act16;
+        m = hull_sample_mask(a_low[slot], a_high[slot], sm.samples, half, margin) & act16;
       }
       const unsigned lb = unit_ballot(m != 0u);
       if (m) {
         const int slot = (qb_h + qb_n + __popc(lb & below)) & (kSlots - 1);
         b_id[slot] = cid;
         b_pos[slot] = cpos;
-        b_mask[slot] = m;
+        b_mask[slot] = (uint16_t)m;
       }
       qa_h = (qa_h + take_a) & (kSlots - 1);
       qa_n -= take_a;
       qb_n += __popc(lb);
       __syncwarp();
     }
-    // the staged records have landed; up to two later copies of hull lines may still be on their way
-    if (since == 0) cp_async_wait<0>(); else if (since == 1) cp_async_wait<1>(); else cp_async_wait<2>();
+    // the staged records have landed; up to kAhead later copies of hull lines may still be on their way
+    static_assert(kAhead == 3, "one case for each number of later copies that may leave those of the records on their way");
+    if (since == 0) cp_async_wait<0>(); else if (since == 1) cp_async_wait<1>(); else if (since == 2) cp_async_wait<2>();
     __syncwarp();
     // ---- stage 3a: evaluate the batch staged one round ago; every lane walks the entries covering its pixel
     uint32_t bits = (active && n_cur > 0) ? __brev(transpose_masks(batch_mask + (second ? kBatch : 0), lane16)) : 0u;  // entry j: bit 31 - j
@@ -988,7 +1025,7 @@ __device__ __forceinline__ void walk_unit(
         if (mine) {
           const uint32_t bit = 0x80000000u >> j;
           mine ^= bit;
-          const float4* rec = stage + j * kStageStride;
+          const float4* rec = stage + j * kStride;
           const float4 pl[4] = {rec[0], rec[1], rec[2], rec[3]};
           const float4 cg = rec[4], cb = rec[5];
           if (slab_test(pl, ray, min_t, cb.w, e)) {
@@ -1041,9 +1078,9 @@ __device__ __forceinline__ void walk_unit(
       while (bits > floor) {
         const int b = 31 - __clz(bits), j = 31 - b;
         bits ^= 1u << b;
-        const float4* rec = stage + j * kStageStride;
+        const float4* rec = stage + j * kStride;
         const float4 pl[4] = {rec[0], rec[1], rec[2], rec[3]};
-        const float4 cg = rec[4], cb = rec[5];
+        const float4 cg = rec[4], cb = rec[kStride == 5 ? 4 : 5];
         Eval e;
         if (slab_test(pl, ray, min_t, cb.w, e)) {
           if (MODE == kStats) {
@@ -1137,7 +1174,7 @@ __device__ __forceinline__ void walk_unit(
       }
     }
     if (MODE == kColor && hit_ids && n_cur > 0) {  // append the batch to the hit list
-      const int64_t hslot = sm.hits[half][0] + n_ent + el, mslot = sm.hits[half][1] + n_ent + el;
+      const int64_t hslot = sm.hits(half)[0] + n_ent + el, mslot = sm.hits(half)[1] + n_ent + el;
       if (el < n_cur && RM_INDEX_OK(hslot, RM_X_HIT_IDS, 2)) {
         const int id = batch_id[el];
         hit_ids[hslot] = id;
@@ -1156,16 +1193,23 @@ __device__ __forceinline__ void walk_unit(
     uint32_t mask = 0;
     if (el < take) {
       const int slot = (qb_h + el) & (kSlots - 1);
-      const int id = b_id[slot];
-      batch_id[el] = id;
+      batch_id[el] = b_id[slot];
       batch_pos[el] = b_pos[slot];
       mask = b_mask[slot];
-      const float4* src_rec = records + record_at(id);
-      float4* dst = stage + el * kStageStride;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) cp_async16(dst + k, src_rec + k);
     }
-    batch_mask[el] = mask;
+    batch_mask[(el & 16) + 2 * (el & 7) + ((el >> 3) & 1)] = (uint16_t)mask;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {  // two lanes for the record of an entry
+      const int e = (el >> 1) + k * (kEntries / 2);
+      if (e < take) {
+        const float4* src_rec = records + record_at(b_id[(qb_h + e) & (kSlots - 1)]) + (el & 1);
+        float4* dst = stage + e * kStride + (el & 1);
+        cp_async16(dst, src_rec);
+        cp_async16(dst + 2, src_rec + 2);
+        if (kStride == 7) cp_async16(dst + 4, src_rec + 4);
+        else if (el & 1) cp_async16(dst + 3, src_rec + 4);  // density; the colours are not staged
+      }
+    }
     cp_async_commit();
     since = 0;
     qb_h = (qb_h + take) & (kSlots - 1);
@@ -1215,9 +1259,8 @@ k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, con
 }
 
 // Long first: the first `long_blocks` of the grid take the tiles whose list is longer than `long_list`.
-// 92 registers, as the walk by halves takes in a kernel of its own.  Two warps per block: the same time at 2M tets, with four
-// 1 % more at 6M and 1.7 % at 18M.
-constexpr int kLongFirstWarps = 2;
+// 92 registers, as the walk by halves takes in a kernel of its own.  Blocks of two warps would leave 18 of them on an SM, of four 20.
+constexpr int kLongFirstWarps = 4;
 __global__ void __maxnreg__(92)
 k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
                      const float2* __restrict__ jitter, float4* __restrict__ out_img, float* __restrict__ dist_img,
