@@ -1379,34 +1379,29 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   const int64_t unit = ((int64_t)blockIdx.x * kBwdWarps<PAIR> + warp) * (PAIR ? 1 : 2) + half;
   Unit u = make_unit(rcam, ranges, unit, n_units, subs, lane16);
 
-  f3 d = {0.f, 0.f, 1.f};
+  // The half-warp's hit list (written by the forward pass: the batches of 16 it evaluated, each with its tet ids
+  // and, per pixel, the bit set of the batch entries the pixel hit).  Round k takes entries [n c, n c + n) with
+  // n = kEntries, c = rounds - 1 - k.  Its first loads come before the pixel's, which they do not depend on.
+  const int64_t unit_at = (int64_t)u.tile * u.subs + u.sub;
+  int nmax = (unit < n_units && RM_INDEX_OK(unit_at, RM_X_UNITS, 4)) ? __ldg(hit_counts + unit_at) : 0;
   const int64_t pix = (int64_t)u.y * rcam.image_width + u.x;
+  float2 at_pixel = make_float2(0.5f, 0.5f);
   float logT = 0.f, sz = 0.f, sw = 0.f;
-  float gr = 0.f, gg = 0.f, gb = 0.f, glogT = 0.f, gx2 = 0.f, gy2 = 0.f, gz = 0.f, gw = 0.f, gv = 0.f;
+  float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float gx2 = 0.f, gy2 = 0.f, gz = 0.f, gw = 0.f, gv = 0.f;
   if (u.inside) {
-    float2 j = jitter ? __ldg(jitter + pix) : make_float2(0.5f, 0.5f);
-    d = ray_direction(rcam, (float)u.x + j.x, (float)u.y + j.y);
+    if (jitter) at_pixel = __ldg(jitter + pix);
     logT = __ldg(out_img + pix).w;
     sz = __ldg(dist_img + 5 * pix + 2);
     sw = __ldg(dist_img + 5 * pix + 3);
-    float4 g4 = __ldg(g_img + pix);
-    gr = g4.x; gg = g4.y; gb = g4.z; glogT = g4.w;
+    g4 = __ldg(g_img + pix);
     const float* gd = g_dist + 5 * pix;
     gx2 = 2.0f * __ldg(gd); gy2 = 2.0f * __ldg(gd + 1); gz = __ldg(gd + 2); gw = __ldg(gd + 3);
     gv = __ldg(gd + 4) * (1.0f / 3.0f);
   }
-  const float G = gr + gg + gb;
-  sm.pixel[lane16][half][0] = make_float4(d.x, d.y, d.z, 1.0f);
-  sm.pixel[lane16][half][1] = make_float4(gr, gg, gb, G);
-  const float min_t = rcam.min_t;
-
-  // The half-warp's hit list (written by the forward pass: the batches of 16 it evaluated, each with its tet ids
-  // and, per pixel, the bit set of the batch entries the pixel hit).  Round k takes entries [n c, n c + n) with
-  // n = kEntries, c = rounds - 1 - k.
   const int64_t hbase = (int64_t)u.start * u.subs + (int64_t)u.sub * u.len;
-  const int64_t mbase = hbase + 16 * ((int64_t)u.tile * u.subs + u.sub);
-  int nmax = (unit < n_units && RM_INDEX_OK((int64_t)u.tile * u.subs + u.sub, RM_X_UNITS, 4))
-                 ? min(__ldg(hit_counts + (int64_t)u.tile * u.subs + u.sub), u.len) : 0;
+  const int64_t mbase = hbase + 16 * unit_at;
+  nmax = min(nmax, u.len);
   if (nmax > 0 && !(RM_INDEX_OK(hbase + nmax - 1, RM_X_HIT_IDS, 2) &&
                     RM_INDEX_OK(mbase + (nmax + kBatch - 1) / kBatch * kBatch - 1, RM_X_HIT_MASKS, 3)))
     nmax = 0;
@@ -1417,15 +1412,20 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   const int ent = (PAIR ? lane : lane16) >> 1, part = lane16 & 1;
   int id_next = 0;         // tet id of `ent` in the round staged next
   unsigned bits_next = 0;  // this pixel's bits of that round
-  auto fetch = [&](int c) {
-    id_next = 0;
+  int c = rounds - 1;      // the round that `fetch` reads
+  const int32_t* id_at = hit_ids + hbase + (int64_t)c * kEntries + ent;
+  const uint16_t* mask_at = hit_masks + mbase + (PAIR ? c : c >> 1) * kBatch + lane16;
+  // The addresses go down by steps; with the address of a round from scratch each time, and the pixel's values before the hit
+  // list's, 2M tets took 2.43 ms, not 2.36, and 21M 3.08, not 2.98.
+  auto fetch = [&](bool whole) {
     bits_next = 0;
     if (c >= 0) {
-      const int e = c * kEntries + ent;
-      if (e < nmax) id_next = __ldg(hit_ids + hbase + e);
-      bits_next = PAIR ? (unsigned)__ldg(hit_masks + mbase + c * kBatch + lane16)
-                       : ((unsigned)__ldg(hit_masks + mbase + (c >> 1) * kBatch + lane16) >> (kBwdBatch * (c & 1))) & 0xFFu;
+      id_next = whole || c * kEntries + ent < nmax ? __ldg(id_at) : 0;
+      bits_next = PAIR ? (unsigned)__ldg(mask_at) : ((unsigned)__ldg(mask_at) >> (kBwdBatch * (c & 1))) & 0xFFu;
       if (!RM_INDEX_OK(id_next, RM_X_TETS, 1)) id_next = 0;
+      if (PAIR || !(c & 1)) mask_at -= kBatch;
+      id_at -= kEntries;
+      --c;
     }
   };
   auto stage = [&](int k) {
@@ -1437,6 +1437,15 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
     }
     cp_async_commit();
   };
+  fetch(false);
+  f3 d = {0.f, 0.f, 1.f};
+  if (u.inside) d = ray_direction(rcam, (float)u.x + at_pixel.x, (float)u.y + at_pixel.y);
+  stage(0);
+  const float gr = g4.x, gg = g4.y, gb = g4.z, G = gr + gg + gb;
+  float glogT = g4.w;
+  sm.pixel[lane16][half][0] = make_float4(d.x, d.y, d.z, 1.0f);
+  sm.pixel[lane16][half][1] = make_float4(gr, gg, gb, G);
+  const float min_t = rcam.min_t;
   const Ray ray = make_ray(d);
   // what phase A leaves of a hit: an entering distance te <= 0 is clamped and has no gradient
   auto leave = [&](int j, const Crossing& cr, float te, float g_enter, float g_exit, float a, float b, float w) {
@@ -1447,12 +1456,10 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   };
   float4* const faces_row = staged + ent * kBwdStageStride + kFacesAt;
   if (part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
-  fetch(rounds - 1);
-  stage(0);
   for (int k = 0; k < max_rounds; ++k) {
     unsigned bits = bits_next;
     const int id = id_next;  // of the entry this lane sums
-    fetch(rounds - 2 - k);
+    fetch(true);
     cp_async_wait<0>();
     __syncwarp();
 
