@@ -1448,6 +1448,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   sm.pixel[lane16][half][1] = make_float4(gr, gg, gb, G);
   const float min_t = rcam.min_t;
   const Ray ray = make_ray(d);
+  const float gx = 0.5f * gx2;
   // what phase A leaves of a hit: an entering distance te <= 0 is clamped and has no gradient
   auto leave = [&](int j, const Crossing& cr, float te, float g_enter, float g_exit, float a, float b, float w) {
     const float q_e = te > 0.0f ? -g_enter * cr.r_e : 0.0f, q_x = -g_exit * cr.r_x;
@@ -1531,43 +1532,39 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
       const float4 cg = rec[4], cb = rec[5];
       const Crossing cr = slab_planes(pl, ray);
       // A hit has entered before it leaves and leaves in front of the origin, so the leaving distance needs no
-      // clamp.  (The forward pass found the optical depth positive with the same operations; the test only keeps
+      // clamp.  (The forward pass found the optical depth positive with the same operations; the clamp only keeps
       // a disagreement from dividing by zero.)
       const float te = cr.ue - min_t, exit = cr.ux - min_t;
       const float enter = fmaxf(te, 0.0f), dens = cb.w;
-      const float dt = exit - enter, tau = dens * dt;
-      if (tau > 0.0f) {
-        const float X = exit + min_t, E = enter + min_t;
-        const float gd = cg.x * d.x + cg.y * d.y + cg.z * d.z;
-        const float oe = fmaf(E, gd, cg.w), ox = fmaf(X, gd, cg.w);
-        float alpha, w0, w1, slope;
-        segment_weights(tau, alpha, w0, w1, slope);
-        // undo: state before this tet
-        logT += tau;
-        const float Tp = fast_exp(fminf(logT, 46.0517f));
-        const float mid = (exit + enter) * 0.5f, m1 = dens * mid;
-        sz -= dens;
-        sw -= m1;
-        // reverse of the state update
-        const float g_m1 = fmaf(sz, gx2, gw), g_m0 = fmaf(sw, gy2, gz);
-        const float w = w0 + w1;
-        const float gcb = gr * cb.x + gg * cb.y + gb * cb.z;  // colour of the tet against the upstream gradient
-        const float g_a = -glogT;
-        glogT = fmaf(fmaf(w, gcb, fmaf(w0, ox, w1 * oe) * G), Tp, glogT);
-        gz = fmaf(m1, gx2, gz);
-        gw = fmaf(dens, gy2, gw);
-        // reverse of the segment integral
-        const float TG = Tp * G, TC = Tp * gcb;
-        const float g_ox = w0 * TG, g_oe = w1 * TG;
-        // d w0 / d tau = alpha + d phi / d tau, d w1 / d tau = -d phi / d tau, d phi / d tau = -slope
-        const float g_tau = fmaf(TG * (oe - ox), slope, fmaf(fmaf(TG, ox, TC), alpha, g_a));
-        const float gvd = gv * dens;
-        const float b = fmaf(fmaf(2.0f, gvd, g_tau), dt, fmaf(g_m1, mid, g_m0));
-        const float g_dt = fmaf(gvd, dens, g_tau * dens), g_mid = 0.5f * g_m1 * dens;
-        const float g_exit = fmaf(g_ox, gd, g_mid) + g_dt, g_enter = fmaf(g_oe, gd, g_mid) - g_dt;
-        // planes: t = u - min_t, u = -D/den  =>  dt/dD = -1/den, dt/dn = -u/den d
-        leave(j, cr, te, g_enter, g_exit, fmaf(g_ox, X, g_oe * E), b, w * Tp);
-      }
+      const float dt = exit - enter, tau = fmaxf(dens * dt, 1e-30f);
+      const float X = cr.ux, E = fmaxf(cr.ue, min_t);
+      const float gd = cg.x * d.x + cg.y * d.y + cg.z * d.z;
+      const float oe = fmaf(E, gd, cg.w), ox = fmaf(X, gd, cg.w);
+      float alpha, w0, w1, slope;
+      segment_weights(tau, alpha, w0, w1, slope);
+      // undo: state before this tet
+      logT += tau;
+      const float Tp = fast_exp(fminf(logT, 46.0517f));
+      const float sum = exit + enter, m1x2 = dens * sum;  // twice the first moment
+      // reverse of the state update
+      sz -= dens;
+      sw = fmaf(-0.5f, m1x2, sw);
+      const float g_m1 = fmaf(sz, gx2, gw), g_m0 = fmaf(sw, gy2, gz);
+      gw = fmaf(dens, gy2, gw);
+      gz = fmaf(m1x2, gx, gz);
+      const float gcb = gr * cb.x + gg * cb.y + gb * cb.z;  // colour of the tet against the upstream gradient
+      // reverse of the segment integral
+      const float TG = Tp * G, TC = Tp * gcb, w = w0 + w1;
+      const float g_ox = w0 * TG, g_oe = w1 * TG;
+      // d w0 / d tau = alpha + d phi / d tau, d w1 / d tau = -d phi / d tau, d phi / d tau = -slope
+      const float g_tau = fmaf(TG * (oe - ox), slope, fmaf(fmaf(TG, ox, TC), alpha, -glogT));
+      glogT += fmaf(w, TC, fmaf(g_ox, ox, g_oe * oe));
+      const float gvd = gv * dens, half_m1 = 0.5f * g_m1;
+      const float b = fmaf(fmaf(2.0f, gvd, g_tau), dt, fmaf(half_m1, sum, g_m0));
+      const float g_dt = fmaf(gvd, dens, g_tau * dens), g_mid = half_m1 * dens;
+      const float g_exit = fmaf(g_ox, gd, g_mid) + g_dt, g_enter = fmaf(g_oe, gd, g_mid) - g_dt;
+      // planes: t = u - min_t, u = -D/den  =>  dt/dD = -1/den, dt/dn = -u/den d
+      leave(j, cr, te, g_enter, g_exit, fmaf(g_ox, X, g_oe * E), b, w * Tp);
     }
     __syncwarp();
     // the entry's face bytes and the signs of its two planes' -D, before the copies of the next round and its phase A write there
