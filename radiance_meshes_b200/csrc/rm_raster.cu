@@ -640,7 +640,7 @@ __device__ __forceinline__ SampleBox halfwarp_sample_box(bool inside, float2 s, 
 // A half-warp owns 16 pixels of one tile and walks the tile's list in three stages that
 // are decoupled by two small queues in shared memory (ring buffers of 32 slots):
 //   1. examination, 16 entries at a time: every lane tests the hull lines of one entry
-//      (32 bytes, on their way to shared memory three steps ahead, their tet ids as many
+//      (32 bytes, on their way to shared memory two steps ahead, their tet ids as many
 //      before that) against the bounding box of the half-warp's samples (k_pack_records marks
 //      the lines of a tet of zero density); survivors go to queue A in list order with their
 //      position and their lines;
@@ -662,10 +662,12 @@ __device__ __forceinline__ SampleBox halfwarp_sample_box(bool inside, float2 s, 
 constexpr int kBatch = 16;       // entries staged and evaluated per half-warp and round
 constexpr int kRing = 32;        // slots of each candidate queue
 // Examination steps whose hull lines are on their way; tet ids are read as many steps before that.  A step is 100 instructions and
-// waited 1,360 cycles for its ids and lines, as did stage 2 for its lines, when these were read one step ahead and from L1: 2M tets,
-// 822 x 1237, 2.01 ms, 6.7M, 1080p, 1.83, 36M, 2160p, 7.39, constant colour, 600k, 800 x 800, 0.54; now 1.78, 1.63, 6.67, 0.52, of
-// which the order of a step (copies before the test) is 2 %.  Before, 59 % of the issue slots; now 70 %, with 4 % more instructions.
-constexpr int kAhead = 3;
+// waited 1,360 cycles for its ids and lines, as did stage 2 for its lines, when lines and ids were fetched a step later each and
+// stage 2 read its lines from L1: 2M tets, 822 x 1237, 2.01 ms, 6.7M, 1080p, 1.83, 36M, 2160p, 7.39, constant colour, 600k,
+// 800 x 800, 0.54; now 1.80, 1.65, 6.72, 0.52, of which the order of a step (copies before the test) is 2 %.  Before, 59 % of the
+// issue slots; now 70 %, with 4 % more instructions.  Three steps instead of two are no faster on large grids and leave less of
+// L1 (600k, 800 x 800: 377 us with two, 385 with three) and two warps less of the statistics (2M: 2.35 ms and 2.47).
+constexpr int kAhead = 2;
 
 // An examination step on its way: hull lines of its entries, first and second 16 bytes apart by a distance at which two lanes
 // that copy the two of one entry meet no bank twice, and tet ids, of this step and of the one kAhead later in turn.
@@ -674,7 +676,7 @@ struct ExamStep {
   int ids[2][32];
 };
 // What a warp keeps in shared memory.  What the evaluation loop does not need - hull lines on their way to the
-// examination, sample box, hit-list positions - lives here and not in registers.  11.4 KB: five blocks of four warps per SM.
+// examination, sample box, hit-list positions - lives here and not in registers.  10 KB: five blocks of four warps per SM.
 template <int STRIDE>
 struct WalkShared {
   float4 stage[2 * kBatch * STRIDE];
@@ -898,8 +900,8 @@ __device__ __forceinline__ void walk_unit(
   bool fetching = act16 != 0;
   int n_ent = 0;  // entries in the hit list
 
-  // Examination: entry src + el is the one this lane examines next.  The hull lines of that step and of the two behind it are
-  // in sm.steps or on their way, and so are the tet ids of the three steps behind those.  All of it by asynchronous copies, two
+  // Examination: entry src + el is the one this lane examines next.  The hull lines of that step and of the kAhead - 1 behind it
+  // are in sm.steps or on their way, and so are the tet ids of the kAhead steps behind those.  All of it by asynchronous copies, two
   // lanes for the lines of an entry, so that a sector is one access.  Behind the end of the list its last entry is copied.
   int src = 0;
   int qa_h = 0, qa_n = 0, qb_h = 0, qb_n = 0;  // ring heads and fill levels (the same in all lanes of the half)
@@ -999,7 +1001,7 @@ __device__ __forceinline__ void walk_unit(
       __syncwarp();
     }
     // the staged records have landed; up to kAhead later copies of hull lines may still be on their way
-    static_assert(kAhead == 3, "one case for each number of later copies that may leave those of the records on their way");
+    static_assert(kAhead <= 3, "one case for each number of later copies that may leave those of the records on their way");
     if (since == 0) cp_async_wait<0>(); else if (since == 1) cp_async_wait<1>(); else if (since == 2) cp_async_wait<2>();
     __syncwarp();
     // ---- stage 3a: evaluate the batch staged one round ago; every lane walks the entries covering its pixel
