@@ -1416,15 +1416,14 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
   int id_next = 0;         // tet id of `ent` in the round staged next
   unsigned bits_next = 0;  // this pixel's bits of that round
   int c = rounds - 1;      // the round that `fetch` reads
-  const int32_t* id_at = hit_ids + hbase + (int64_t)c * kEntries + ent;
-  const uint16_t* mask_at = hit_masks + mbase + (PAIR ? c : c >> 1) * kBatch + lane16;
-  // The addresses go down by steps; with the address of a round from scratch each time, and the pixel's values before the hit
+  int64_t id_at = hbase + (int64_t)c * kEntries + ent, mask_at = mbase + (int64_t)(PAIR ? c : c >> 1) * kBatch + lane16;
+  // The places go down by steps; with those of a round from scratch each time, and the pixel's values before the hit
   // list's, 2M tets took 2.43 ms, not 2.36, and 21M 3.08, not 2.98.
   auto fetch = [&](bool whole) {
     bits_next = 0;
     if (c >= 0) {
-      id_next = whole || c * kEntries + ent < nmax ? __ldg(id_at) : 0;
-      bits_next = PAIR ? (unsigned)__ldg(mask_at) : ((unsigned)__ldg(mask_at) >> (kBwdBatch * (c & 1))) & 0xFFu;
+      id_next = whole || c * kEntries + ent < nmax ? __ldg(hit_ids + id_at) : 0;
+      bits_next = PAIR ? (unsigned)__ldg(hit_masks + mask_at) : ((unsigned)__ldg(hit_masks + mask_at) >> (kBwdBatch * (c & 1))) & 0xFFu;
       if (!RM_INDEX_OK(id_next, RM_X_TETS, 1)) id_next = 0;
       if (PAIR || !(c & 1)) mask_at -= kBatch;
       id_at -= kEntries;
