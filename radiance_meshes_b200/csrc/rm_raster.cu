@@ -677,17 +677,16 @@ struct ExamStep {
 };
 // What a warp keeps in shared memory.  What the evaluation loop does not need - hull lines on their way to the
 // examination, sample box, hit-list positions - lives here and not in registers.  10 KB: five blocks of four warps per SM.
-template <int STRIDE>
+template <int STRIDE, bool POSITIONS>
 struct WalkShared {
   float4 stage[2 * kBatch * STRIDE];
   ExamStep steps[kAhead];                  // [step % kAhead]; the gap of the first two: what `box` and `hits` return
   float4 a_low[2 * kRing], a_high[2 * kRing];  // hull lines of the entries in queue A
   float4 samples[8][2];                    // [pair][half]: two samples each: x0, x1, y0, y1
   uint16_t batch_mask[2 * kBatch];         // entries e and e + 8 of 16 in one word
-  int a_id[2 * kRing], a_pos[2 * kRing];
-  int b_id[2 * kRing], b_pos[2 * kRing];
+  int a_id[2 * kRing], b_id[2 * kRing], batch_id[2 * kBatch];
   uint16_t b_mask[2 * kRing];
-  int batch_id[2 * kBatch], batch_pos[2 * kBatch];
+  int a_pos[POSITIONS ? 2 * kRing : 1], b_pos[POSITIONS ? 2 * kRing : 1], batch_pos[POSITIONS ? 2 * kBatch : 1];
 
   __device__ __forceinline__ float4* box(int half) { return &steps[0].gap[2 * half]; }  // centre and half extents, then the margin
   __device__ __forceinline__ int64_t* hits(int half) {  // first id slot and first mask slot of the hit list
@@ -758,19 +757,24 @@ __device__ __forceinline__ uint32_t transpose_masks(const uint16_t* __restrict__
 // per (entry, half row) then adds them up over the 16 pixels, multiplied by constants of the pixel, and issues
 // one or three 128-bit reductions.  2M tets, 822 x 1237, a lens: 3.62 ms for a walk of its own over the entries in
 // lock-step with 16 sums by shuffles, 2.60 ms for sums pixel by pixel with what was not hit masked out, 2.51 ms for sums of
-// two pixels in a packed addition, a slot of zeros in the place of what was not hit.
+// two pixels in a packed addition, a slot of zeros in the place of what was not hit.  Then
+// a lane per (entry, half row) that adds up all 16 pixels with selections took 2.35 ms, with predicates on the multiply-adds 2.30.
 enum ForwardMode { kColor, kConstColor, kStats };
 constexpr int kStatsBatch = 8;  // entries whose hits are in shared memory at a time
 
 // float4 per staged record: 6 used, of the statistics, which need no colours, 5; the odd stride spreads the records over the banks
 template <ForwardMode MODE>
 constexpr int kStageStride = MODE == kStats ? 5 : 7;
-using FwdShared = WalkShared<kStageStride<kColor>>;
-struct StatsShared : WalkShared<kStageStride<kStats>> {
-  float4 hit[2 * kStatsBatch * 16 + 1];  // [half, entry_slot]: T, T * entry distance, T * exit distance; the last one: zeros
-  float4 pixel[3][4][2][2];              // [component][four pixels][0: err, err^2, ssim; 1: ray direction][half]
+using FwdShared = WalkShared<kStageStride<kColor>, true>;
+// What a hit leaves, at [pixel] of its entry's row: for part 0 of the sums T twice, for part 1 T times its two distances.  The odd
+// stride in units of 16 bytes spreads the entries over the banks.
+struct StatsRow {
+  float4 hit[16], unused;
 };
-constexpr int kNoHit = 2 * kStatsBatch * 16;
+struct StatsShared : WalkShared<kStageStride<kStats>, false> {  // 13.8 KB; nobody asks for the number of entries walked
+  StatsRow rows[2 * kStatsBatch];
+  float4 pixel[16][2][2];  // [pixel][half][part]: err, err^2, ssim, 1; ray direction, its x again
+};
 struct StatsArgs {
   const float *pixel_err, *ssim_err;
   float* tet_err;
@@ -790,9 +794,6 @@ struct StatsArgs {
 //               1.88 -> 1.64 ms; 18M: 3.27 -> 2.49 ms).
 // A pixel's hits are taken in the same order with the same operations in all of them: which one a call uses cannot be told
 // from the bits of its image, so that a frame in bands, each dealt by its own size, is the frame.
-// Slot of (entry, pixel): the exclusive-or spreads the accesses by pixel and by entry over the banks.
-__device__ __forceinline__ int entry_slot(int e, int p) { return e * 16 + (p ^ e); }
-
 // A pixel's state behind a hit: transmittance and distortion moments (dy without a factor of two, dv without one of a third).
 // m2: twice the first moment of the density over the segment; of the constant-colour variant the laddered distance.
 template <ForwardMode MODE>
@@ -884,12 +885,8 @@ __device__ __forceinline__ void walk_unit(
       perr = __ldg(stats.pixel_err + pix);
       serr = __ldg(stats.ssim_err + pix);
     }
-    const float con[2][3] = {{perr, perr * perr, serr}, {d.x, d.y, d.z}};
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int w = 0; w < 2; ++w) reinterpret_cast<float*>(&sm.pixel[c][lane16 >> 2][w][half])[lane16 & 3] = con[w][c];
-    if (lane == 0) sm.hit[kNoHit] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sm.pixel[lane16][half][0] = make_float4(perr, perr * perr, serr, 1.0f);
+    sm.pixel[lane16][half][1] = make_float4(d.x, d.y, d.z, d.x);
   }
 
   float sr = 0.f, sg = 0.f, sb = 0.f, logT = MODE == kStats ? 1.0f : 0.0f, T = MODE == kStats ? 2.718281828f : 1.0f;
@@ -968,7 +965,7 @@ __device__ __forceinline__ void walk_unit(
         if (cand) {
           const int slot = (qa_h + qa_n + __popc(cb & below)) & (kSlots - 1);
           a_id[slot] = id;
-          a_pos[slot] = pos;
+          if (MODE != kStats) a_pos[slot] = pos;
           a_low[slot] = l0;
           a_high[slot] = l1;
         }
@@ -984,7 +981,7 @@ __device__ __forceinline__ void walk_unit(
       if (el < take_a) {
         const int slot = (qa_h + el) & (kSlots - 1);
         cid = a_id[slot];
-        cpos = a_pos[slot];
+        if (MODE != kStats) cpos = a_pos[slot];
         const float margin = rcam.camera_type == 1 ? kFisheyeMargin : kPixelMargin;
         m = hull_sample_mask(a_low[slot], a_high[slot], sm.samples, half, margin) & act16;
       }
@@ -992,7 +989,7 @@ __device__ __forceinline__ void walk_unit(
       if (m) {
         const int slot = (qb_h + qb_n + __popc(lb & below)) & (kSlots - 1);
         b_id[slot] = cid;
-        b_pos[slot] = cpos;
+        if (MODE != kStats) b_pos[slot] = cpos;
         b_mask[slot] = (uint16_t)m;
       }
       qa_h = (qa_h + take_a) & (kSlots - 1);
@@ -1097,7 +1094,7 @@ __device__ __forceinline__ void walk_unit(
           bool finished;
           if constexpr (MODE == kStats) {
             const float Tw = T * e.tau;
-            sm.hit[half * kStatsBatch * 16 + entry_slot(j & 7, lane16)] = make_float4(Tw, Tw * (e.enter + min_t), Tw * (e.exit + min_t), 0.0f);
+            sm.rows[half * kStatsBatch + (j & 7)].hit[lane16] = make_float4(Tw, Tw, Tw * (e.enter + min_t), Tw * (e.exit + min_t));
             logT -= e.tau;
             T *= e.alpha;
             finished = logT < -5.5f;
@@ -1108,7 +1105,7 @@ __device__ __forceinline__ void walk_unit(
           }
           if (finished) {
             active = false;
-            contrib = batch_pos[j] + 1;  // entries walked, the terminating one included
+            if (MODE != kStats) contrib = batch_pos[j] + 1;  // entries walked, the terminating one included
             hitbits ^= bits;
             bits = 0;
           }
@@ -1127,36 +1124,31 @@ __device__ __forceinline__ void walk_unit(
           if (ent == e) mine = col;
         }
         mine = (mine >> (16 * half)) & 0xFFFFu;
-        // a pixel that has not hit the entry is read from the slot of zeros; two pixels in a packed addition
-        float2 sums[7];
+        // part 0: v = (T, T), x, y, z its sums with err, err^2 and ssim, u without; part 1: v = T times the two distances, x, y, z
+        // and u, v, w their sums with the ray direction.  Even and odd pixels apart: two short sums are rounded less than a long one.
+        struct Sums { float x, y, z, u, v, w, most; } sums[2];
+        sums[0] = sums[1] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const float2* const row = reinterpret_cast<const float2*>(sm.rows[half * kStatsBatch + ent].hit) + part;
 #pragma unroll
-        for (int i = 0; i < 7; ++i) sums[i] = make_float2(0.f, 0.f);
-        float most = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int first = half * kStatsBatch * 16 + ent * 16;
-          float4 con[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) con[c] = sm.pixel[c][q][part][half];
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const int p = 4 * q + 2 * t;
-            const float4 h0 = sm.hit[(mine >> p) & 1u ? first + (p ^ ent) : kNoHit];
-            const float4 h1 = sm.hit[(mine >> p) & 2u ? first + ((p + 1) ^ ent) : kNoHit];
-            const float2 w = {h0.x, h1.x}, f1 = part ? make_float2(h0.y, h1.y) : w, f2 = {h0.z, h1.z};
-            sums[0] = add2(sums[0], w);
-            most = fmaxf(most, fmaxf(w.x, w.y));
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const float2 two = t ? make_float2(con[c].z, con[c].w) : make_float2(con[c].x, con[c].y);
-              sums[1 + c] = fma2(f1, two, sums[1 + c]);
-              sums[4 + c] = fma2(f2, two, sums[4 + c]);
-            }
-          }
+        for (int p = 0; p < 16; ++p) {
+          const float4 con = sm.pixel[p][half][part];
+          const float2 v = row[2 * p];
+          Sums& t = sums[p & 1];
+          asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+              "and.b32 t, %7, %8;\n\tsetp.ne.u32 p, t, 0;\n\t"
+              "@p fma.rn.f32 %0, %9, %11, %0;\n\t"
+              "@p fma.rn.f32 %1, %9, %12, %1;\n\t"
+              "@p fma.rn.f32 %2, %9, %13, %2;\n\t"
+              "@p fma.rn.f32 %3, %10, %14, %3;\n\t"
+              "@p fma.rn.f32 %4, %10, %12, %4;\n\t"
+              "@p fma.rn.f32 %5, %10, %13, %5;\n\t"
+              "@p max.f32 %6, %6, %9;\n\t}"
+              : "+f"(t.x), "+f"(t.y), "+f"(t.z), "+f"(t.u), "+f"(t.v), "+f"(t.w), "+f"(t.most)
+              : "r"(mine), "r"(1u << p), "f"(v.x), "f"(v.y), "f"(con.x), "f"(con.y), "f"(con.z), "f"(con.w));
         }
-        auto total = [&](int i) { return sums[i].x + sums[i].y; };
-        const float sum = total(0);
-        const f3 s1 = {total(1), total(2), total(3)}, s2 = {total(4), total(5), total(6)};
+        const f3 s1 = {sums[0].x + sums[1].x, sums[0].y + sums[1].y, sums[0].z + sums[1].z};
+        const f3 s2 = {sums[0].u + sums[1].u, sums[0].v + sums[1].v, sums[0].w + sums[1].w};
+        const float most = fmaxf(sums[0].most, sums[1].most), sum = __shfl_sync(FULL, s2.x, lane & ~1);  // part 0's
         const float ssim = __shfl_xor_sync(FULL, s1.z, 1);  // part 0's, needed in a row that part 1 writes
         if (mine) {
           const int64_t id = batch_id[8 * sub + ent];
@@ -1197,7 +1189,7 @@ __device__ __forceinline__ void walk_unit(
     if (el < take) {
       const int slot = (qb_h + el) & (kSlots - 1);
       batch_id[el] = b_id[slot];
-      batch_pos[el] = b_pos[slot];
+      if (MODE != kStats) batch_pos[el] = b_pos[slot];
       mask = b_mask[slot];
     }
     batch_mask[(el & 16) + 2 * (el & 7) + ((el >> 3) & 1)] = (uint16_t)mask;
