@@ -13,24 +13,27 @@ from delaunay_rasterization.internal.tile_shader_slang import lookup_tiles_touch
 from radiance_meshes_b200 import _lib, raster
 
 
+def _pack(indices, vertices, rgbs, cam, tiles_touched):
+    """(cell values, records) of the interpolating renderer with a zero colour gradient: (density, r, g, b, 0, 0, 0)."""
+    rgbs = rgbs.detach().float()
+    assert rgbs.shape[1] == 4, "rgbs are (r, g, b, density) per tet"
+    cell = torch.cat([rgbs[:, 3:4], rgbs[:, :3], torch.zeros((indices.shape[0], 3), device=vertices.device)], dim=1).contiguous()
+    return cell, raster.pack_records(indices, vertices.detach().contiguous().float(), cell, cam, tiles_touched)
+
+
 class AlphaBlendTiledRender(torch.autograd.Function):
     """apply(sorted_tetra_idx, tile_ranges, indices, vertices, rgbs[T,4] = (r,g,b,density), render_grid, tcam,
     pre_multi, ladder_p) -> (output_img[H,W,4] = (r,g,b,transmittance), distortion_img[H,W,4])."""
 
     @staticmethod
-    def forward(ctx, sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, pre_multi, ladder_p,
-                device="cuda"):
+    def forward(ctx, sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, pre_multi, ladder_p, *extra):
+        # extra: the reference's optional `device` argument, then what _pack has returned for these arguments
+        ctx.n_extra = len(extra)
         dev = vertices.device
         raster._require_cuda(vertices, "vertices")
         cam = raster.CameraArgs(tcam, dev)
         assert cam.c.grid_height == render_grid.grid_height and cam.c.grid_width == render_grid.grid_width
-        rgbs = rgbs.detach().float()
-        assert rgbs.shape[1] == 4, "rgbs are (r, g, b, density) per tet"
-        T = indices.shape[0]
-        # records of the interpolating renderer with a zero colour gradient: (density, r, g, b, 0, 0, 0)
-        cell = torch.cat([rgbs[:, 3:4], rgbs[:, :3], torch.zeros((T, 3), device=dev)], dim=1).contiguous()
-        records = raster.pack_records(indices, vertices.detach().contiguous().float(), cell, cam,
-                                      lookup_tiles_touched(sorted_tetra_idx))
+        cell, records = extra[1] if len(extra) > 1 else _pack(indices, vertices, rgbs, cam, lookup_tiles_touched(sorted_tetra_idx))
         H, W = render_grid.image_height, render_grid.image_width
         lib = _lib.load()
         with torch.cuda.device(dev):
@@ -72,7 +75,7 @@ class AlphaBlendTiledRender(torch.autograd.Function):
                 raster._ptr(grad_records), raster._ptr(flags), raster._ptr(vertices_grad), raster._ptr(cell_grad),
                 raster._stream(dev)))
         rgbs_grad = torch.cat([cell_grad[:, 1:4], cell_grad[:, 0:1]], dim=1)
-        return None, None, None, vertices_grad, rgbs_grad, None, None, None, None
+        return (None, None, None, vertices_grad, rgbs_grad, None, None, None, None) + (None,) * ctx.n_extra
 
 
 def render_constant_color(indices, vertices, rgbs_fn, camera, cell_values=None, tile_size=16, min_t=0.1):
@@ -86,11 +89,15 @@ def render_constant_color(indices, vertices, rgbs_fn, camera, cell_values=None, 
     render_grid = RenderGrid(camera.image_height, camera.image_width, tile_height=tile_size, tile_width=tile_size)
     tcam = dict(tile_height=tile_size, tile_width=tile_size, grid_height=render_grid.grid_height,
                 grid_width=render_grid.grid_width, min_t=min_t, **camera.to_dict(device))
-    sorted_tetra_idx, tile_ranges, vs_tetra, circumcenter, mask, _ = vertex_and_tile_shader(
-        indices, vertices, tcam, render_grid)
     rgbs = cell_values
+    packed = []  # the records, packed while the host waits for the number of list entries
+
+    def pack(bctx):
+        packed.append(_pack(indices, vertices, rgbs, bctx["cam"], bctx["tiles_touched"]))
+    sorted_tetra_idx, tile_ranges, vs_tetra, circumcenter, mask, _ = vertex_and_tile_shader(
+        indices, vertices, tcam, render_grid, pack)
     image_rgb, distortion_img = AlphaBlendTiledRender.apply(
-        sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, 100, -0.1)
+        sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, 100, -0.1, "cuda", packed[0])
     return {
         "render": image_rgb.permute(2, 0, 1)[:3, ...],
         "viewspace_points": vs_tetra,

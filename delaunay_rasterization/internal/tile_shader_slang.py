@@ -50,11 +50,15 @@ class VertexShader(torch.autograd.Function):
         return (None, grad_vertices, None, None) + (None,) * ctx.n_extra
 
 
-def vertex_and_tile_shader(indices, vertices, cam, render_grid):
+def vertex_and_tile_shader(indices, vertices, cam, render_grid, before_wait=None):
+    """`before_wait(bctx)`, if given, is called when the projection is enqueued, before the host waits for the number of list
+    entries: what it enqueues runs while the host learns that number and enqueues the list build."""
     holder = {}
     tiles_touched, rect_tile_space, vs_tetra, circumcenter = VertexShader.apply(indices, vertices, cam, render_grid,
                                                                                 "cuda", holder)
     bctx = holder.pop("bctx")
+    if before_wait is not None:
+        before_wait(bctx)
     n_keys, _ = raster.read_info(bctx)
     sorted_tetra_idx = raster.build_tile_lists(bctx, n_keys)
     sorted_tetra_idx._rm_tiles_touched = tiles_touched

@@ -7,6 +7,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
@@ -117,21 +118,30 @@ struct Camera {
   }
 };
 
-// A copy of a frame's info block in page-locked memory, which the device writes once the stream is there.  The memory goes
-// back only after that, also where a frame is given up in between: it would otherwise be somebody else's by then.
+// A copy of a frame's info block in page-locked memory, which the device has written once the stream has passed `written`.  The
+// memory goes back only after that, also where a frame is given up in between: it would otherwise be somebody else's by then.
 struct PendingInfo {
   Tensor block;
+  at::cuda::CUDAEvent written;
   c10::cuda::CUDAStream stream;
-  bool arrived = false;
+  bool recorded = false, arrived = false;
 
   explicit PendingInfo(c10::cuda::CUDAStream s)
       : block(at::empty({3}, at::TensorOptions().dtype(at::kLong).pinned_memory(true))), stream(s) {}
   ~PendingInfo() {
     if (!arrived) cudaStreamSynchronize(stream.stream());
   }
-  // The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).
+  void record() {
+    written.record(stream);
+    recorded = true;
+  }
+  // The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).  What was enqueued behind
+  // the info block is not waited for.
   std::tuple<int64_t, int64_t, int64_t, int64_t> wait() {
-    if (!arrived) stream.synchronize();
+    if (!arrived) {
+      if (recorded) written.synchronize();
+      else stream.synchronize();
+    }
     arrived = true;
     const RmBinInfo* r = ptr<RmBinInfo>(block);
     return {r->n_keys, r->n_region_keys, r->n_visible, r->status};
@@ -161,6 +171,7 @@ std::tuple<std::vector<Tensor>, std::unique_ptr<PendingInfo>> project_and_bin(co
                                        ptr<int32_t>(tile_ranges), ptr<RmBinInfo>(info), workspace.data_ptr(), bytes,
                                        ptr<uint8_t>(visible), pending ? ptr<RmBinInfo>(pending->block) : nullptr,
                                        stream_of(vertices)));
+  if (pending) pending->record();
   std::vector<Tensor> out = {indices, vertices, tiles_touched, rect, vs_tetra, circumcenter, tile_ranges, info, workspace,
                              visible};
   return {std::move(out), std::move(pending)};
@@ -227,12 +238,9 @@ std::vector<Tensor> forward(const Tensor& list, const Tensor& tile_ranges, const
   return out;
 }
 
-// Everything AlphaBlendTiledRender.forward does.  Returns (output_img, distortion_img, tet_alive, indices, vertices, cell,
-// records, n_contributors, tet_flags[, counts, ids, masks]); the bracketed ones if need_grad.
-std::vector<Tensor> blend_forward(const Tensor& list, const Tensor& tile_ranges, const Tensor& indices_in,
-                                  const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address, bool zero_fill,
-                                  const c10::optional<Tensor>& jitter_in, const c10::optional<Tensor>& tiles_touched,
-                                  bool need_grad) {
+// What blend_forward does before its walk: (tet_alive, indices, vertices, cell, records[, tet_flags]); the last one if need_grad.
+std::vector<Tensor> pack_for_blend(const Tensor& indices_in, const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address,
+                                   const c10::optional<Tensor>& tiles_touched, bool need_grad) {
   require_cuda(vertices_in, "vertices");
   const at::Device dev = vertices_in.device();
   c10::cuda::CUDAGuard guard(dev);
@@ -240,12 +248,29 @@ std::vector<Tensor> blend_forward(const Tensor& list, const Tensor& tile_ranges,
   const int64_t T = indices.size(0);
   // tet_alive is never written by the reference kernel either: always False
   Tensor tet_alive = empty({T}, at::kBool, dev);
-  c10::optional<Tensor> flags, jitter;
+  c10::optional<Tensor> flags;
   if (need_grad) flags = empty({std::max<int64_t>(T, 1)}, at::kByte, dev);
-  if (jitter_in.has_value()) jitter = f32(*jitter_in);
   Tensor records = pack_records(indices, vertices, cell, cam_address, tiles_touched, tet_alive, flags);
-  std::vector<Tensor> f = forward(list, tile_ranges, records, cam_address, zero_fill, jitter, flags);
-  std::vector<Tensor> out = {f[0], f[1], tet_alive, indices, vertices, cell, records, f[2]};
+  std::vector<Tensor> out = {tet_alive, indices, vertices, cell, records};
+  if (need_grad) out.push_back(*flags);
+  return out;
+}
+
+// Everything AlphaBlendTiledRender.forward does.  Returns (output_img, distortion_img, tet_alive, indices, vertices, cell,
+// records, n_contributors, tet_flags[, counts, ids, masks]); the bracketed ones if need_grad.  packed: what pack_for_blend has
+// returned for the same arguments.
+std::vector<Tensor> blend_forward(const Tensor& list, const Tensor& tile_ranges, const Tensor& indices_in,
+                                  const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address, bool zero_fill,
+                                  const c10::optional<Tensor>& jitter_in, const c10::optional<Tensor>& tiles_touched,
+                                  bool need_grad, const c10::optional<std::vector<Tensor>>& packed) {
+  const std::vector<Tensor> p =
+      packed.has_value() ? *packed : pack_for_blend(indices_in, vertices_in, cell_in, cam_address, tiles_touched, need_grad);
+  c10::cuda::CUDAGuard guard(vertices_in.device());
+  c10::optional<Tensor> flags, jitter;
+  if (need_grad) flags = p.at(5);
+  if (jitter_in.has_value()) jitter = f32(*jitter_in);
+  std::vector<Tensor> f = forward(list, tile_ranges, p[4], cam_address, zero_fill, jitter, flags);
+  std::vector<Tensor> out = {f[0], f[1], p[0], p[1], p[2], p[3], p[4], f[2]};
   if (need_grad) {
     out.push_back(*flags);
     out.insert(out.end(), f.begin() + 3, f.end());
@@ -317,7 +342,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("build_tile_lists", &build_tile_lists, unlocked);
   m.def("pack_records", &pack_records, unlocked);
   m.def("forward", &forward, unlocked);
+  m.def("pack_for_blend", &pack_for_blend, unlocked);
   m.def("blend_forward", &blend_forward, unlocked);
+  m.def("blend_forward", [](const Tensor& list, const Tensor& tile_ranges, const Tensor& indices, const Tensor& vertices,
+                            const Tensor& cell, uintptr_t cam, bool zero_fill, const c10::optional<Tensor>& jitter,
+                            const c10::optional<Tensor>& tiles_touched, bool need_grad) {
+    return blend_forward(list, tile_ranges, indices, vertices, cell, cam, zero_fill, jitter, tiles_touched, need_grad, c10::nullopt);
+  }, unlocked);
   m.def("backward", &backward, unlocked);
   m.def("distortion_loss", &distortion_loss, unlocked);
   m.def("distortion_loss_backward", &distortion_loss_backward, unlocked);

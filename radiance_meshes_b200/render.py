@@ -3,7 +3,7 @@
 uses them (utils/train_util.py:14-75), for given per-tet cell values."""
 import torch
 
-from delaunay_rasterization.internal.alphablend_tiled_slang_interp import AlphaBlendTiledRender
+from delaunay_rasterization.internal.alphablend_tiled_slang_interp import AlphaBlendTiledRender, pack_ahead
 from delaunay_rasterization.internal.render_grid import RenderGrid
 from delaunay_rasterization.internal.tile_shader_slang import vertex_and_tile_shader
 from radiance_meshes_b200 import _lib
@@ -45,12 +45,19 @@ def render(indices, vertices, cell_values, tcam, ray_jitter=None, before_blend=N
     reads `cell_values` and `ray_jitter` is launched (a pipeline waits there for their copies to land)."""
     H, W = int(tcam["image_height"]), int(tcam["image_width"])
     grid = RenderGrid(H, W, tile_height=int(tcam["tile_height"]), tile_width=int(tcam["tile_width"]))
+    packed = []
+
+    def pack(bctx):
+        packed.append(pack_ahead(bctx, indices, vertices, cell_values))
+    # Where the cell values are there already, the records are packed while the host waits for the number of list entries and
+    # enqueues the list build; the device has nothing else to do then (60k tets, 203 x 317: 179 -> 170 us).
     sorted_tetra_idx, tile_ranges, vs_tetra, circumcenter, mask, rect = vertex_and_tile_shader(
-        indices, vertices, tcam, grid)
+        indices, vertices, tcam, grid, pack if before_blend is None else None)
     if before_blend is not None:
         before_blend()
     image, distortion_img, tet_alive = AlphaBlendTiledRender.apply(
-        sorted_tetra_idx, tile_ranges, indices, vertices, cell_values, grid, tcam, ray_jitter)
+        sorted_tetra_idx, tile_ranges, indices, vertices, cell_values, grid, tcam, ray_jitter, "cuda",
+        packed[0] if packed else None)
     return dict(render=image.permute(2, 0, 1)[:3], alpha=image[..., 3], distortion_loss=DistortionLoss.apply(distortion_img),
                 mask=mask, image=image, distortion_img=distortion_img, sorted_tetra_idx=sorted_tetra_idx,
                 tile_ranges=tile_ranges, vs_tetra=vs_tetra, circumcenter=circumcenter, rect=rect)
