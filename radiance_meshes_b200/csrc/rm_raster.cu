@@ -582,6 +582,21 @@ struct Unit {
   int sub, subs;  // which 16-pixel group of the tile this half-warp owns, out of how many
 };
 
+// The t-th tile to be walked: rows in pairs, tiles of a pair in blocks of 2 x 2, so that the warps of a block have a patch of
+// tiles and not a strip, with fewer tets on its border (6.7M tets, 1080p, forward 1.64 -> 1.60 ms, backward 1.80 -> 1.77; 36M,
+// 2160p, 6.72 -> 6.62; 21M backward 2.92 -> 2.88; the others the same.  Patches of 4 x 2, 4 x 4 and 8 x 4 give less).
+__device__ __forceinline__ int walked_tile(const RmCamera& c, int64_t t) {
+  const unsigned width = c.grid_width, rows = c.tile_row_end - c.tile_row_begin;
+  const unsigned pair = (unsigned)t / (2 * width), r = (unsigned)t - pair * 2 * width, even = width & ~1u;
+  unsigned x = r, y = 2 * pair;
+  if (y + 1 < rows) {
+    const bool block = r < 2 * even;
+    x = block ? 2 * (r >> 2) + (r & 1u) : width - 1;
+    y += block ? (r >> 1) & 1u : r - 2 * even;
+  }
+  return (int)((c.tile_row_begin + y) * width + x);
+}
+
 __device__ __forceinline__ Unit make_unit(const RmCamera& c, const int2* __restrict__ ranges, int64_t unit,
                                           int64_t n_units, int subs, int lane16) {
   Unit u;
@@ -595,7 +610,7 @@ __device__ __forceinline__ Unit make_unit(const RmCamera& c, const int2* __restr
   if (unit >= n_units) return u;
   int64_t t = unit / subs;
   int sub = (int)(unit - t * subs);
-  u.tile = c.tile_row_begin * c.grid_width + (int)t;
+  u.tile = walked_tile(c, t);
   int ty = u.tile / c.grid_width, tx = u.tile - ty * c.grid_width;
   u.sub = sub;
   int lx, ly;
@@ -1270,10 +1285,9 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
   const int64_t walkers = (int64_t)long_blocks * kLongFirstWarps;
   int64_t at = (int64_t)blockIdx.x * kLongFirstWarps + warp;
   if (at < walkers) {
-    const int first = rcam.tile_row_begin * rcam.grid_width;
     for (; at < n_units; at += 32 * walkers) {
       const int64_t u = at + lane * walkers;
-      const int2 rg = u < n_units ? __ldg(ranges + first + u / subs) : make_int2(0, 0);
+      const int2 rg = u < n_units ? __ldg(ranges + walked_tile(rcam, u / subs)) : make_int2(0, 0);
       unsigned found = __ballot_sync(0xffffffffu, rg.y - rg.x > long_list);
       while (found) {
         const int64_t unit = at + (__ffs(found) - 1) * walkers;
