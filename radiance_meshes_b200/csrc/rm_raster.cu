@@ -835,7 +835,8 @@ template <ForwardMode MODE>
 using ForwardShared = typename std::conditional<MODE == kStats, StatsShared, FwdShared>::type;
 
 // The walk of one unit (PAIR), or of the two units of a warp's halves.  Lists longer than `skip_length` are left to others.
-template <ForwardMode MODE, bool PAIR>
+// PAST_L1: hull lines are copied past L1; the rule is at lines_past_l1.
+template <ForwardMode MODE, bool PAIR, bool PAST_L1>
 __device__ __forceinline__ void walk_unit(
     ForwardShared<MODE>& sm, int64_t unit, int skip_length, const int32_t* __restrict__ list,
     const int2* __restrict__ ranges, const float4* __restrict__ records, const RmCamera& rcam,
@@ -929,7 +930,9 @@ __device__ __forceinline__ void walk_unit(
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int id = st->ids[at][pair_lane + k * (kEntries / 2)];
-      if (RM_INDEX_OK(id, RM_X_TETS, 1)) cp_async16_l1(to + k * (kEntries / 2), lines_at + record_at(id));
+      if (!RM_INDEX_OK(id, RM_X_TETS, 1)) continue;
+      if (PAST_L1) cp_async16(to + k * (kEntries / 2), lines_at + record_at(id));
+      else cp_async16_l1(to + k * (kEntries / 2), lines_at + record_at(id));
     }
     cp_async4(&st->ids[at ^ 1][lane], list_at + min(first + kAhead * kEntries + el, last));
   };
@@ -1253,7 +1256,7 @@ __device__ __forceinline__ void walk_unit(
 // count (600k tets, 800 x 800, pairs: 416 us with four, 435 with two, 469 with one).
 template <ForwardMode MODE>
 constexpr int kFwdWarps = MODE == kStats ? 2 : kWarpsPerBlock;
-template <ForwardMode MODE, bool PAIR>
+template <ForwardMode MODE, bool PAIR, bool PAST_L1>
 __global__ void __launch_bounds__(kFwdWarps<MODE> * 32, (MODE == kStats ? 16 : 20) / kFwdWarps<MODE>)
 k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
           const float2* __restrict__ jitter, float4* __restrict__ out_img, float* __restrict__ dist_img,
@@ -1263,7 +1266,7 @@ k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, con
   extern __shared__ __align__(16) unsigned char smem_fwd[];
   const int warp = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
   const int64_t at = (int64_t)blockIdx.x * kFwdWarps<MODE> + warp;
-  walk_unit<MODE, PAIR>(reinterpret_cast<ForwardShared<MODE>*>(smem_fwd)[warp], PAIR ? at : 2 * at + half, INT_MAX, list, ranges,
+  walk_unit<MODE, PAIR, PAST_L1>(reinterpret_cast<ForwardShared<MODE>*>(smem_fwd)[warp], PAIR ? at : 2 * at + half, INT_MAX, list, ranges,
                         records, rcam, jitter, out_img, dist_img, n_contrib, hit_counts, hit_ids, hit_masks, tet_flags, subs,
                         n_units, pre_multi, ladder_p, stats);
 }
@@ -1271,6 +1274,7 @@ k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, con
 // Long first: the first `long_blocks` of the grid take the tiles whose list is longer than `long_list`.
 // 92 registers, as the walk by halves takes in a kernel of its own.  Blocks of two warps would leave 18 of them on an SM, of four 20.
 constexpr int kLongFirstWarps = 4;
+template <bool PAST_L1>
 __global__ void __maxnreg__(92)
 k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ ranges, const float4* __restrict__ records, RmCamera rcam,
                      const float2* __restrict__ jitter, float4* __restrict__ out_img, float* __restrict__ dist_img,
@@ -1292,7 +1296,7 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
       while (found) {
         const int64_t unit = at + (__ffs(found) - 1) * walkers;
         found &= found - 1;
-        walk_unit<kColor, true>(sm, unit, INT_MAX, list, ranges, records, rcam, jitter, out_img, dist_img, n_contrib, hit_counts,
+        walk_unit<kColor, true, PAST_L1>(sm, unit, INT_MAX, list, ranges, records, rcam, jitter, out_img, dist_img, n_contrib, hit_counts,
                                 hit_ids, hit_masks, tet_flags, subs, n_units, 0.0f, 0.0f, StatsArgs{});
         __syncwarp();
       }
@@ -1300,7 +1304,7 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
     return;
   }
   at = (int64_t)(blockIdx.x - (unsigned)long_blocks) * kLongFirstWarps + warp;
-  walk_unit<kColor, false>(sm, at * 2 + (lane >> 4), long_list, list, ranges, records, rcam, jitter, out_img, dist_img, n_contrib,
+  walk_unit<kColor, false, PAST_L1>(sm, at * 2 + (lane >> 4), long_list, list, ranges, records, rcam, jitter, out_img, dist_img, n_contrib,
                            hit_counts, hit_ids, hit_masks, tet_flags, subs, n_units, 0.0f, 0.0f, StatsArgs{});
 }
 
@@ -2005,6 +2009,13 @@ static bool deal_by_pairs(int64_t n_units, int64_t tiles, int64_t n_list) {
   return n_units <= 2 * kWave || (n_units <= 8 * kWave && n_list >= 64 * tiles);
 }
 
+// Whether hull lines are copied past L1: where lists have 800 entries on average, those of the tiles that an SM walks at a time name
+// more lines than L1 holds (50 KB, and a line of it for each sector), and filling it costs more than the hits save (forward, average
+// list: 3M tets of a scene, 300 x 300, 2742: 1049 us through L1, 846 past it; 6.7M, 600 x 600, 1634: 736, 627; 21M, 1080p, 1886:
+// 2166, 2024; 6.7M, 1080p, 1083: 1518, 1501; 1.2M in clusters, 300 x 300, 909: 304, 291).  Short lists live of it (0.6M, 800 x 800,
+// 230: 375, 414; 1.2M, 600 x 600, 415: 400, 459); between 650 and 880 it is the same.
+static bool lines_past_l1(int64_t tiles, int64_t n_list) { return n_list >= 800 * tiles; }
+
 int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* records, const RmCamera* cam,
                       const float* jitter, float* out_img, float* dist_img, int32_t* n_contrib, const RmHitList* hits,
                       int64_t n_list, cudaStream_t st) {
@@ -2027,12 +2038,14 @@ int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* r
     constexpr int warps = rm::kLongFirstWarps, long_blocks = 148 * 20 / warps;
     const int long_list = (int)std::min<int64_t>(3 * n_list / tiles, INT_MAX);
     blocks = (unsigned)((n_units + 2 * warps - 1) / (2 * warps));
-    RM_CUDA_CHECK(rm_launch(rm::k_forward_long_first, blocks + long_blocks, warps * 32, warps * sizeof(rm::FwdShared), st, list, tiles_list, recs, *cam,
+    auto kernel = lines_past_l1(tiles, n_list) ? rm::k_forward_long_first<true> : rm::k_forward_long_first<false>;
+    RM_CUDA_CHECK(rm_launch(kernel, blocks + long_blocks, warps * 32, warps * sizeof(rm::FwdShared), st, list, tiles_list, recs, *cam,
                             jit, img, dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, long_list,
                             long_blocks));
   } else {
     const bool pair = deal_by_pairs(n_units, tiles, n_list);
-    auto kernel = pair ? rm::k_forward<rm::kColor, true> : rm::k_forward<rm::kColor, false>;
+    auto kernel = !pair ? rm::k_forward<rm::kColor, false, false>
+                  : lines_past_l1(tiles, n_list) ? rm::k_forward<rm::kColor, true, true> : rm::k_forward<rm::kColor, true, false>;
     RM_CUDA_CHECK(rm_launch(kernel, pair ? pair_blocks : blocks, threads, smem, st, list, tiles_list, recs, *cam, jit, img,
                             dist_img, n_contrib, h.counts, h.ids, h.masks, h.tet_flags, subs, n_units, 0.0f, 0.0f,
                             rm::StatsArgs{}));
@@ -2051,7 +2064,7 @@ int rm_launch_forward_constant_color(const int32_t* list, const int32_t* ranges,
   RmProfScope prof("k_forward<constant colour>", st);
   const bool pair = deal_by_pairs(n_units, n_units / subs, n_list);
   if (pair) blocks = (unsigned)((n_units + rm::kWarpsPerBlock - 1) / rm::kWarpsPerBlock);
-  auto kernel = pair ? rm::k_forward<rm::kConstColor, true> : rm::k_forward<rm::kConstColor, false>;
+  auto kernel = pair ? rm::k_forward<rm::kConstColor, true, false> : rm::k_forward<rm::kConstColor, false, false>;
   RM_CUDA_CHECK(rm_launch(kernel, blocks, rm::kWarpsPerBlock * 32, rm::kWarpsPerBlock * sizeof(rm::FwdShared), st, list,
                           reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
                           reinterpret_cast<float4*>(out_img), dist_img, n_contrib, nullptr, nullptr, nullptr, nullptr, subs,
@@ -2097,10 +2110,10 @@ int rm_launch_tet_err(const int32_t* list, const int32_t* ranges, const float* r
   unit_grid(cam, warps, &subs, &n_units, &blocks);
   if (n_units == 0) return RM_OK;
   constexpr size_t smem = warps * sizeof(rm::StatsShared);
-  RM_CUDA_CHECK(cudaFuncSetAttribute(rm::k_forward<rm::kStats, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  RM_CUDA_CHECK(cudaFuncSetAttribute(rm::k_forward<rm::kStats, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   RmProfScope prof("k_tet_err", st);
-  RM_CUDA_CHECK(rm_launch(rm::k_forward<rm::kStats, false>, blocks, warps * 32, smem, st, list,
+  RM_CUDA_CHECK(rm_launch(rm::k_forward<rm::kStats, false, false>, blocks, warps * 32, smem, st, list,
                           reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(records), *cam, nullptr,
                           nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, subs, n_units, 0.0f, 0.0f,
                           rm::StatsArgs{pixel_err, ssim_err, tet_err, tet_count}));
