@@ -14,25 +14,19 @@ from delaunay_rasterization.internal.tile_shader_slang import lookup_tiles_touch
 from radiance_meshes_b200 import _lib, raster
 
 
-def _need_grad(vertices, tet_density):
-    return vertices.requires_grad or tet_density.requires_grad
-
-
 def pack_ahead(bctx, indices, vertices, tet_density):
-    """The records of a frame whose projection is enqueued, packed before its tile lists are built, for the last argument of
+    """(camera, records) of a frame whose projection is enqueued, packed before its tile lists are built, for the last argument of
     AlphaBlendTiledRender.apply; None where the arguments are not such as that takes."""
-    if not (isinstance(tet_density, torch.Tensor) and tet_density.is_cuda and tet_density.device == vertices.device and
-            tet_density.shape == (indices.shape[0], 7)):
-        return None
-    return _lib.native().pack_for_blend(indices, vertices, tet_density, bctx["cam"].address, bctx["tiles_touched"],
-                                        _need_grad(vertices, tet_density))
+    cam = bctx["cam"]
+    packed = _lib.native().pack_ahead(indices, vertices, tet_density, cam.address, bctx["tiles_touched"])
+    return None if packed is None else (cam, packed)
 
 
 class AlphaBlendTiledRender(torch.autograd.Function):
     @staticmethod
     def forward(ctx, sorted_tetra_idx, tile_ranges, indices, vertices, tet_density, render_grid, tcam, ray_jitter, *extra):
         # extra: the reference's optional `device` argument, then what pack_ahead has returned for these arguments
-        packed = extra[1] if len(extra) > 1 else None
+        cam, packed = extra[1] if len(extra) > 1 and extra[1] is not None else (None, None)
         ctx.n_extra = len(extra)
         assert tet_density.shape[1] == 7, "cell values are (density, r, g, b, gx, gy, gz) per tet"
         if ray_jitter is not None:  # None: the pixel centres
@@ -41,9 +35,10 @@ class AlphaBlendTiledRender(torch.autograd.Function):
                 # once for both directions: the caller may refill a jitter that was copied as soon as this returns
                 ray_jitter = ray_jitter.detach().float().contiguous()
         raster._require_cuda(vertices, "vertices")
-        cam = raster.CameraArgs(tcam, vertices.device)
+        if cam is None:
+            cam = raster.CameraArgs(tcam, vertices.device)
         assert cam.native.grid == (render_grid.grid_height, render_grid.grid_width)
-        need_grad = _need_grad(vertices, tet_density)
+        need_grad = vertices.requires_grad or tet_density.requires_grad
         out = _lib.native().blend_forward(sorted_tetra_idx, tile_ranges, indices, vertices, tet_density, cam.address,
                                           cam.native.zero_fill, ray_jitter, lookup_tiles_touched(sorted_tetra_idx),
                                           need_grad, packed)

@@ -679,8 +679,8 @@ constexpr int kRing = 32;        // slots of each candidate queue
 // Examination steps whose hull lines are on their way; tet ids are read as many steps before that.  A step is 100 instructions and
 // waited 1,360 cycles for its ids and lines, as did stage 2 for its lines, when lines and ids were fetched a step later each and
 // stage 2 read its lines from L1: 2M tets, 822 x 1237, 2.01 ms, 6.7M, 1080p, 1.83, 36M, 2160p, 7.39, constant colour, 600k,
-// 800 x 800, 0.54; now 1.80, 1.65, 6.72, 0.52, of which the order of a step (copies before the test) is 2 %.  Before, 59 % of the
-// issue slots; now 70 %, with 4 % more instructions.  Three steps instead of two are no faster on large grids and leave less of
+// 800 x 800, 0.54; then 1.80, 1.65, 6.72, 0.52, of which the order of a step (copies before the test) is 2 % (1.59 and 6.50 with
+// tiles in blocks and lines past L1, below).  Before, 59 % of the issue slots; now 70 %, with 3 % more instructions.  Three steps instead of two are no faster on large grids and leave less of
 // L1 (600k, 800 x 800: 377 us with two, 385 with three) and two warps less of the statistics (2M: 2.35 ms and 2.47).
 constexpr int kAhead = 2;
 
@@ -1334,8 +1334,9 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
 // (u = -D / den, so q u = dL/dt u^2 / D, and without the reciprocals, whose pick by plane costs six instructions a hit, 2M tets
 // would take 2.33 ms; but the sums, divided by D at the end, are 3 % further from 64 bits.)
 // With selections in phase B and 8 ballots a round for who has hit what: 2M tets, 822 x 1237,
-// 2.70 ms, 6.7M, 1080p, 2.14, 21M 3.61, a medium scene 1.04e9 warp instructions; now 2.43, 1.92, 3.07 ms, 0.9e9.  (A lock-step walk
-// over the entries with a reduction per step took twice that.)
+// 2.70 ms, 6.7M, 1080p, 2.14, 21M 3.61, a medium scene 1.04e9 warp instructions; then 2.43, 1.92, 3.07 ms, 0.9e9; 2.28, 1.77,
+// 2.88 and 0.87e9 with fewer instructions per hit, the hit list's loads first, tiles in blocks.  (A lock-step walk over the entries
+// with a reduction per step took twice that.)
 constexpr int kBwdBatch = 8;          // entries per half-warp and round
 constexpr int kBwdStageStride = 7;    // float4 per staged record (6 used), as in the forward kernel
 
@@ -1771,7 +1772,8 @@ k_clear_flagged_rows(const uint8_t* __restrict__ tet_flags, int64_t T, float4* _
 // vertices and by the atomics, on which all lanes of a warp are with a list, 20 of 32 with a tet per lane.  Warps wait for
 // nobody: a list and rows of the whole block of 64 threads, PER = 4, cost meshes with a gradient in every tet more than a
 // thread per tet did (1.05M 92.5 us -> 94.5, 2M in random order 168 -> 175; now 90.5 and 171).  Scenes with a thread per tet in
-// blocks of 256: 2M 78 us, 6.7M 252, 21M 595; now 62, 187 and 353.
+// blocks of 256: 2M 78 us, 6.7M 252, 21M 595; with lists 62, 187 and 353; with two reductions a vertex for three 54 and 162, and
+// another view of the 21M scene 548 -> 494.
 constexpr int kFinishThreads = 64;
 
 template <int PER>
@@ -1852,8 +1854,7 @@ k_backward_finish(const int32_t* __restrict__ indices, const float* __restrict__
     gvv[0] = gvv[0] - grd * gs0;
   #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      // the two of a vertex's three floats that begin on 8 bytes in one reduction: two instead of three a vertex (6.7M tets
-      // 187 -> 162 us, 21M 548 -> 494)
+      // the two of a vertex's three floats that begin on 8 bytes in one reduction
       float* vp = vgrad + 3 * (int64_t)vid[k];
       const bool late = reinterpret_cast<uintptr_t>(vp) & 4;
       atomicAdd(reinterpret_cast<float2*>(vp + (late ? 1 : 0)), late ? make_float2(gvv[k].y, gvv[k].z) : make_float2(gvv[k].x, gvv[k].y));

@@ -238,8 +238,12 @@ std::vector<Tensor> forward(const Tensor& list, const Tensor& tile_ranges, const
   return out;
 }
 
-// What blend_forward does before its walk: (tet_alive, indices, vertices, cell, records[, tet_flags]); the last one if need_grad.
-std::vector<Tensor> pack_for_blend(const Tensor& indices_in, const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address,
+// What blend_forward does before its walk; tet_flags if need_grad.
+struct Packed {
+  Tensor tet_alive, indices, vertices, cell, records;
+  c10::optional<Tensor> tet_flags;
+};
+Packed pack_for_blend(const Tensor& indices_in, const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address,
                                    const c10::optional<Tensor>& tiles_touched, bool need_grad) {
   require_cuda(vertices_in, "vertices");
   const at::Device dev = vertices_in.device();
@@ -251,28 +255,36 @@ std::vector<Tensor> pack_for_blend(const Tensor& indices_in, const Tensor& verti
   c10::optional<Tensor> flags;
   if (need_grad) flags = empty({std::max<int64_t>(T, 1)}, at::kByte, dev);
   Tensor records = pack_records(indices, vertices, cell, cam_address, tiles_touched, tet_alive, flags);
-  std::vector<Tensor> out = {tet_alive, indices, vertices, cell, records};
-  if (need_grad) out.push_back(*flags);
-  return out;
+  return {tet_alive, indices, vertices, cell, records, flags};
+}
+
+// The same ahead of a blend of these arguments; nothing where they are not such as it takes.
+std::unique_ptr<Packed> pack_ahead(const Tensor& indices, const Tensor& vertices, const Tensor& cell, uintptr_t cam_address,
+                                   const Tensor& tiles_touched) {
+  if (!cell.is_cuda() || cell.device() != vertices.device() || cell.dim() != 2 || cell.size(0) != indices.size(0) ||
+      cell.size(1) != 7)
+    return nullptr;
+  return std::make_unique<Packed>(pack_for_blend(indices, vertices, cell, cam_address, tiles_touched,
+                                                 vertices.requires_grad() || cell.requires_grad()));
 }
 
 // Everything AlphaBlendTiledRender.forward does.  Returns (output_img, distortion_img, tet_alive, indices, vertices, cell,
-// records, n_contributors, tet_flags[, counts, ids, masks]); the bracketed ones if need_grad.  packed: what pack_for_blend has
+// records, n_contributors, tet_flags[, counts, ids, masks]); the bracketed ones if need_grad.  packed: what pack_ahead has
 // returned for the same arguments.
 std::vector<Tensor> blend_forward(const Tensor& list, const Tensor& tile_ranges, const Tensor& indices_in,
                                   const Tensor& vertices_in, const Tensor& cell_in, uintptr_t cam_address, bool zero_fill,
                                   const c10::optional<Tensor>& jitter_in, const c10::optional<Tensor>& tiles_touched,
-                                  bool need_grad, const c10::optional<std::vector<Tensor>>& packed) {
-  const std::vector<Tensor> p =
-      packed.has_value() ? *packed : pack_for_blend(indices_in, vertices_in, cell_in, cam_address, tiles_touched, need_grad);
+                                  bool need_grad, const Packed* packed) {
+  const Packed p =
+      packed ? *packed : pack_for_blend(indices_in, vertices_in, cell_in, cam_address, tiles_touched, need_grad);
+  if (need_grad != p.tet_flags.has_value()) throw std::runtime_error("rm_b200: records packed for another kind of blend");
   c10::cuda::CUDAGuard guard(vertices_in.device());
-  c10::optional<Tensor> flags, jitter;
-  if (need_grad) flags = p.at(5);
+  c10::optional<Tensor> jitter;
   if (jitter_in.has_value()) jitter = f32(*jitter_in);
-  std::vector<Tensor> f = forward(list, tile_ranges, p[4], cam_address, zero_fill, jitter, flags);
-  std::vector<Tensor> out = {f[0], f[1], p[0], p[1], p[2], p[3], p[4], f[2]};
+  std::vector<Tensor> f = forward(list, tile_ranges, p.records, cam_address, zero_fill, jitter, p.tet_flags);
+  std::vector<Tensor> out = {f[0], f[1], p.tet_alive, p.indices, p.vertices, p.cell, p.records, f[2]};
   if (need_grad) {
-    out.push_back(*flags);
+    out.push_back(*p.tet_flags);
     out.insert(out.end(), f.begin() + 3, f.end());
   }
   return out;
@@ -342,12 +354,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("build_tile_lists", &build_tile_lists, unlocked);
   m.def("pack_records", &pack_records, unlocked);
   m.def("forward", &forward, unlocked);
-  m.def("pack_for_blend", &pack_for_blend, unlocked);
+  py::class_<Packed>(m, "Packed");
+  m.def("pack_ahead", &pack_ahead, unlocked);
   m.def("blend_forward", &blend_forward, unlocked);
   m.def("blend_forward", [](const Tensor& list, const Tensor& tile_ranges, const Tensor& indices, const Tensor& vertices,
                             const Tensor& cell, uintptr_t cam, bool zero_fill, const c10::optional<Tensor>& jitter,
                             const c10::optional<Tensor>& tiles_touched, bool need_grad) {
-    return blend_forward(list, tile_ranges, indices, vertices, cell, cam, zero_fill, jitter, tiles_touched, need_grad, c10::nullopt);
+    return blend_forward(list, tile_ranges, indices, vertices, cell, cam, zero_fill, jitter, tiles_touched, need_grad, nullptr);
   }, unlocked);
   m.def("backward", &backward, unlocked);
   m.def("distortion_loss", &distortion_loss, unlocked);
