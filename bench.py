@@ -731,7 +731,7 @@ def run_gpu(args):
                         unit="GB/s", frac=(achieved / peak) if achieved else None, traffic=traffic,
                         traffic_source=traffic_src,
                         kernel_ms=kernel_ms[dominant], algorithmic_bytes=bytes_alg,
-                        note="the kernel is bound by instruction issue (ncu: 75 % of the issue slots, DRAM at 5 %), so its HBM "
+                        note="the kernel is bound by instruction issue (ncu: 74 % of the issue slots, DRAM at 6 %), so its HBM "
                              "fraction is low by construction; `fp32_pipe` is its second roofline")
     frame_bytes = sum(alg.values())
     # Second roofline: the integration kernels are bound by instruction issue, not by HBM.  Hits x
