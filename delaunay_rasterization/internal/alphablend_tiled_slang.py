@@ -33,7 +33,8 @@ class AlphaBlendTiledRender(torch.autograd.Function):
         raster._require_cuda(vertices, "vertices")
         cam = raster.CameraArgs(tcam, dev)
         assert cam.c.grid_height == render_grid.grid_height and cam.c.grid_width == render_grid.grid_width
-        cell, records = extra[1] if len(extra) > 1 else _pack(indices, vertices, rgbs, cam, lookup_tiles_touched(sorted_tetra_idx))
+        packed = extra[1] if len(extra) > 1 else None
+        cell, records = packed or _pack(indices, vertices, rgbs, cam, lookup_tiles_touched(sorted_tetra_idx))
         H, W = render_grid.image_height, render_grid.image_width
         lib = _lib.load()
         with torch.cuda.device(dev):
@@ -95,9 +96,10 @@ def render_constant_color(indices, vertices, rgbs_fn, camera, cell_values=None, 
     def pack(bctx):
         packed.append(_pack(indices, vertices, rgbs, bctx["cam"], bctx["tiles_touched"]))
     sorted_tetra_idx, tile_ranges, vs_tetra, circumcenter, mask, _ = vertex_and_tile_shader(
-        indices, vertices, tcam, render_grid, pack)
+        indices, vertices, tcam, render_grid, pack if raster.packs_ahead(indices) else None)
     image_rgb, distortion_img = AlphaBlendTiledRender.apply(
-        sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, 100, -0.1, "cuda", packed[0])
+        sorted_tetra_idx, tile_ranges, indices, vertices, rgbs, render_grid, tcam, 100, -0.1, "cuda",
+        packed[0] if packed else None)
     return {
         "render": image_rgb.permute(2, 0, 1)[:3, ...],
         "viewspace_points": vs_tetra,

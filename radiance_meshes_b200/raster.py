@@ -83,6 +83,19 @@ def build_tile_lists(ctx, n_keys):
                                           ctx.get("n_region_keys", 0))
 
 
+# Up to this many tets the records are packed before the tile lists are built, while the host waits for their length.  They are
+# then alive beside the list scratch (peak of a frame without a backward pass, MB, packed ahead and behind: 1M tets 294 and 240,
+# 2M 900 and 734, 6.7M 2408 and 1920, 36M 13570 and 10720), for the same 7 to 15 us at every size: 60k tets 170.6 us for 180.1,
+# 0.6M 642 for 652, 1M 605 for 612; but 2M 2249 for 2257, 6.7M 2774 for 2788, 36M 14.83 ms for 14.85, within what runs differ by.
+PACK_AHEAD_TETS = 1_000_000
+
+
+def packs_ahead(indices, *differentiable):
+    """Whether to pack ahead.  A frame whose backward pass follows does at any size: its peak is that pass's either way (6.7M tets
+    3416 MB, 21M 8677; 4.64 ms for 4.66 and 8.64 for 8.68)."""
+    return indices.shape[0] <= PACK_AHEAD_TETS or (torch.is_grad_enabled() and any(t.requires_grad for t in differentiable))
+
+
 def pack_records(indices, vertices, cell_values, cam, tiles_touched=None):
     return _lib.native().pack_records(indices, vertices, cell_values, cam.address, tiles_touched, None, None)
 

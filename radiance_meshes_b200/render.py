@@ -6,7 +6,7 @@ import torch
 from delaunay_rasterization.internal.alphablend_tiled_slang_interp import AlphaBlendTiledRender, pack_ahead
 from delaunay_rasterization.internal.render_grid import RenderGrid
 from delaunay_rasterization.internal.tile_shader_slang import vertex_and_tile_shader
-from radiance_meshes_b200 import _lib
+from radiance_meshes_b200 import _lib, raster
 
 
 def tcam_to_device(tcam, device):
@@ -50,9 +50,10 @@ def render(indices, vertices, cell_values, tcam, ray_jitter=None, before_blend=N
     def pack(bctx):
         packed.append(pack_ahead(bctx, indices, vertices, cell_values))
     # Where the cell values are there already, the records are packed while the host waits for the number of list entries and
-    # enqueues the list build; the device has nothing else to do then (60k tets, 203 x 317: 179 -> 170 us).
+    # enqueues the list build; the device has nothing else to do then.
+    ahead = before_blend is None and raster.packs_ahead(indices, vertices, cell_values)
     sorted_tetra_idx, tile_ranges, vs_tetra, circumcenter, mask, rect = vertex_and_tile_shader(
-        indices, vertices, tcam, grid, pack if before_blend is None else None)
+        indices, vertices, tcam, grid, pack if ahead else None)
     if before_blend is not None:
         before_blend()
     image, distortion_img, tet_alive = AlphaBlendTiledRender.apply(

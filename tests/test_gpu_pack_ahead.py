@@ -58,3 +58,59 @@ def test_what_was_refused_stays_refused(cuda_lib, change, error):
     torch.cuda.synchronize()
     good, _, _ = _frame(_inputs(), True, grad=False)  # a frame given up leaves nothing behind
     assert np.isfinite(good["image"].cpu().numpy()).all()
+
+
+def _many_tets(T):
+    """T small tets, among them many copies of the same ones, for a 32 x 32 image."""
+    from radiance_meshes_b200.render import tcam_to_device
+    gen = torch.Generator("cuda").manual_seed(3)
+    v = (4.0 * torch.rand((1024, 1, 3), generator=gen, device="cuda:0") - 2.0 +
+         0.02 * torch.rand((1024, 4, 3), generator=gen, device="cuda:0")).reshape(-1, 3).contiguous()
+    first = 4 * torch.randint(0, 1024, (T, 1), generator=gen, device="cuda:0")
+    return dict(indices=(first + torch.arange(4, device="cuda:0")).to(torch.int32), vertices=v,
+                cell=torch.rand((T, 7), generator=gen, device="cuda:0"), tcam=tcam_to_device(scene_util.camera(H=32, W=32), "cuda:0"),
+                jitter=torch.tensor(scene_util.jitter(32, 32, 5), device="cuda:0"))
+
+
+def _peak(call):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = call()
+    torch.cuda.synchronize()
+    del out
+    return torch.cuda.max_memory_allocated() - before
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_large_mesh_needs_no_more_memory(cuda_lib, grad):
+    """One tet above the limit: records beside the list scratch would be 144 MB more at the peak of a frame alone."""
+    from radiance_meshes_b200 import raster
+    s = _many_tets(raster.PACK_AHEAD_TETS + 1)
+    _frame(s, True, grad)
+    assert _peak(lambda: _frame(s, True, grad)) <= _peak(lambda: _frame(s, False, grad)) + 2**20
+
+
+def test_large_mesh_of_the_constant_colour_renderer_needs_no_more_memory(cuda_lib):
+    from delaunay_rasterization.internal.alphablend_tiled_slang import AlphaBlendTiledRender, render_constant_color
+    from delaunay_rasterization.internal.render_grid import RenderGrid
+    from delaunay_rasterization.internal.tile_shader_slang import vertex_and_tile_shader
+    from radiance_meshes_b200 import raster
+    s = _many_tets(raster.PACK_AHEAD_TETS + 1)
+    rgbs, tcam = s["cell"][:, :4], s["tcam"]
+
+    class camera:
+        image_height = image_width = 32
+        to_dict = staticmethod(lambda device: {k: tcam[k] for k in (
+            "world_view_transform", "K", "cam_pos", "distortion_params", "image_height", "image_width", "fovy", "fovx", "camera_type")})
+
+    def whole():
+        return render_constant_color(s["indices"], s["vertices"], None, camera, cell_values=rgbs, tile_size=4)
+
+    def stages():  # records behind the list build
+        grid = RenderGrid(32, 32, tile_height=4, tile_width=4)
+        ids, ranges, vs, cc, mask, _ = vertex_and_tile_shader(s["indices"], s["vertices"], tcam, grid)
+        return vs, cc, mask, AlphaBlendTiledRender.apply(ids, ranges, s["indices"], s["vertices"], rgbs, grid, tcam, 100, -0.1)
+    whole(), stages()
+    assert _peak(whole) <= _peak(stages) + 2**20
