@@ -14,6 +14,10 @@ def _begin(stream):
     dev = torch.device("cuda:0")
     tcam = tcam_to_device(scene_util.camera(), dev)
     idx, v = torch.tensor(tets, device=dev, dtype=torch.int32), torch.tensor(pts, device=dev)
+    with torch.cuda.stream(stream):
+        # a frame before the one that is looked at: what the first one of a process loads and allocates may take longer than the sleep
+        raster.read_info(raster.project_and_bin(idx, v, tcam, host_info=True))
+        torch.cuda._sleep(1)
     torch.cuda.synchronize()
     with torch.cuda.stream(stream):
         torch.cuda._sleep(100_000_000)  # some 50 ms that the frame waits behind
