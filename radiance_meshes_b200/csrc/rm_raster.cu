@@ -1332,7 +1332,9 @@ k_forward_long_first(const int32_t* __restrict__ list, const int2* __restrict__ 
 //     sign of a plane's D tells.  A lane therefore loads the pair of its plane (8 bytes) and no other, and one bit of the
 //     pixel's byte says whether it counts: a predicate on the multiply-adds, where a selection between both pairs and zero
 //     takes eight instructions a pixel.
-// A near plane behind the camera (BEHIND) has rays that enter and leave on the same side of it: there phase B looks at both pairs.
+// A near plane behind the camera (BEHIND) has rays that enter and leave on the same side of it: the few entries with such hits
+// get a second sum over the other pairs, behind the first (2M tets, min_t = -0.25: 2.33 ms; a second sum for every entry 2.99; 60k
+// 101 and 123 us; the second sum in the first one's registers, which do not hold it, 2.87 ms).
 // (u = -D / den, so q u = dL/dt u^2 / D, and without the reciprocals, whose pick by plane costs six instructions a hit, 2M tets
 // would take 2.33 ms; but the sums, divided by D at the end, are 3 % further from 64 bits.)
 // With selections in phase B and 8 ballots a round for who has hit what: 2M tets, 822 x 1237,
@@ -1586,7 +1588,7 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
     const float2 neg_d = reinterpret_cast<const float2*>(staged + ent * kBwdStageStride + 2 * part + 1)[1];
     const unsigned faces[4] = {__float_as_uint(f4.x), __float_as_uint(f4.y), __float_as_uint(f4.z), __float_as_uint(f4.w)};
     __syncwarp();
-    if (part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!BEHIND && part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
     stage(k + 1);
 
     // ---- phase B: part 0 sums planes 0 and 1, the colour gradient and the density, part 1 planes 2 and 3, the base colour and
@@ -1594,11 +1596,11 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
     const BwdRow& row = rows[ent];
     const float2* const plane_pairs = reinterpret_cast<const float2*>(row.planes);
     const float2* const field_pairs = reinterpret_cast<const float2*>(row.fields) + part;
-    int side0 = neg_d.x < 0.0f ? 0 : 1, side1 = neg_d.y < 0.0f ? 0 : 1;  // entering (facing the camera) or leaving
+    const int side0 = neg_d.x < 0.0f ? 0 : 1, side1 = neg_d.y < 0.0f ? 0 : 1;  // entering (facing the camera) or leaving
     float x0 = 0.f, y0 = 0.f, x1 = 0.f, y1 = 0.f, xf = 0.f, yf = 0.f;
     float2 z0 = {0.f, 0.f}, z1 = z0, zf = z0;
     const unsigned plane0 = 0x01010101u << (4 * part), plane1 = 0x04040404u << (4 * part);
-    unsigned bits0 = plane0 << side0, bits1 = plane1 << side1;
+    const unsigned bits0 = plane0 << side0, bits1 = plane1 << side1;
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
       const unsigned byte = 0xFFu << (8 * (p & 3));
@@ -1607,19 +1609,6 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
       add_where(faces[p >> 2], bits1 & byte, plane_pairs[2 * p + side1], dir.x, dir.y, {dir.z, dir.w}, x1, y1, z1);
       add_where(faces[p >> 2], byte, field_pairs[2 * p], con.x, con.y, {con.z, con.w}, xf, yf, zf);
     }
-    if constexpr (BEHIND) {  // the pairs of the other side
-      side0 ^= 1;
-      side1 ^= 1;
-#pragma unroll 1
-      for (int p = 0; p < 16; ++p) {
-        const unsigned byte = 0xFFu << (8 * (p & 3)), word = reinterpret_cast<const unsigned*>(&f4)[p >> 2];
-        const float4 dir = sm.pixel[p][half][0];
-        add_where(word, (plane0 << side0) & byte, plane_pairs[2 * p + side0], dir.x, dir.y, {dir.z, dir.w}, x0, y0, z0);
-        add_where(word, (plane1 << side1) & byte, plane_pairs[2 * p + side1], dir.x, dir.y, {dir.z, dir.w}, x1, y1, z1);
-      }
-      bits0 = plane0 * 3u;
-      bits1 = plane1 * 3u;
-    }
     const unsigned any = faces[0] | faces[1] | faces[2] | faces[3];
     const float last = __shfl_xor_sync(FULL, zf.y, 1);  // the density's sum belongs to the row of part 1, the offset's to part 0's
     if (any) {
@@ -1627,6 +1616,26 @@ k_backward(const int2* __restrict__ ranges, const float4* __restrict__ records, 
       if (any & bits0) atomicAdd(out + 2 * part, make_float4(x0, y0, z0.x, z0.y));
       if (any & bits1) atomicAdd(out + 2 * part + 1, make_float4(x1, y1, z1.x, z1.y));
       atomicAdd(out + 4 + part, make_float4(xf, yf, zf.x, last));
+    }
+    if constexpr (BEHIND) {  // hits that take a plane from its other side
+      const unsigned other0 = bits0 ^ (3u * plane0), other1 = bits1 ^ (3u * plane1);
+      if (any & (other0 | other1)) {
+        float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+        auto add = [](float4& s, float2 v, float4 dir) {
+          s = make_float4(fmaf(v.x, dir.x, s.x), fmaf(v.x, dir.y, s.y), fmaf(v.x, dir.z, s.z), s.w + v.y);
+        };
+#pragma unroll 1
+        for (int p = 0; p < 16; ++p) {
+          const unsigned face = reinterpret_cast<const uint8_t*>(faces_row)[p];
+          if (face & other0) add(s0, plane_pairs[2 * p + (side0 ^ 1)], sm.pixel[p][half][0]);
+          if (face & other1) add(s1, plane_pairs[2 * p + (side1 ^ 1)], sm.pixel[p][half][0]);
+        }
+        float4* out = reinterpret_cast<float4*>(grec + (int64_t)id * 24);
+        if (any & other0) atomicAdd(out + 2 * part, s0);
+        if (any & other1) atomicAdd(out + 2 * part + 1, s1);
+      }
+      __syncwarp();
+      if (part == 0) *faces_row = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   cp_async_wait<0>();
