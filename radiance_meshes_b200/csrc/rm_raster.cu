@@ -703,6 +703,7 @@ struct WalkShared {
   uint16_t b_mask[2 * kRing];
   int a_pos[POSITIONS ? 2 * kRing : 1], b_pos[POSITIONS ? 2 * kRing : 1], batch_pos[POSITIONS ? 2 * kBatch : 1];
 
+  static_assert(kAhead >= 2, "`hits` are in the gap of the second step");
   __device__ __forceinline__ float4* box(int half) { return &steps[0].gap[2 * half]; }  // centre and half extents, then the margin
   __device__ __forceinline__ int64_t* hits(int half) {  // first id slot and first mask slot of the hit list
     return reinterpret_cast<int64_t*>(&steps[1].gap[half]);
