@@ -1275,7 +1275,8 @@ k_forward(const int32_t* __restrict__ list, const int2* __restrict__ ranges, con
 }
 
 // Long first: the first `long_blocks` of the grid take the tiles whose list is longer than `long_list`.
-// 92 registers, as the walk by halves takes in a kernel of its own.  Blocks of two warps would leave 18 of them on an SM, of four 20.
+// 92 registers, as the walk by halves takes in a kernel of its own.  20 warps fit an SM in blocks of two or of four; with four,
+// neighbouring tiles share more (two and four: 2M tets 1805 and 1793 us, 6.7M 1631 and 1616, 21M 2324 and 2287, 36M 6523 and 6485).
 constexpr int kLongFirstWarps = 4;
 template <bool PAST_L1>
 __global__ void __maxnreg__(92)
@@ -2023,10 +2024,13 @@ static bool deal_by_pairs(int64_t n_units, int64_t tiles, int64_t n_list) {
 }
 
 // Whether hull lines are copied past L1: where lists have 800 entries on average, those of the tiles that an SM walks at a time name
-// more lines than L1 holds (50 KB, and a line of it for each sector), and filling it costs more than the hits save (forward, average
-// list: 3M tets of a scene, 300 x 300, 2742: 1049 us through L1, 846 past it; 6.7M, 600 x 600, 1634: 736, 627; 21M, 1080p, 1886:
-// 2166, 2024; 6.7M, 1080p, 1083: 1518, 1501; 1.2M in clusters, 300 x 300, 909: 304, 291).  Short lists live of it (0.6M, 800 x 800,
-// 230: 375, 414; 1.2M, 600 x 600, 415: 400, 459); between 650 and 880 it is the same.
+// more lines than L1 holds (28 KB beside the walks' shared memory, and a line of it for each sector), and filling it costs more than
+// the hits save (forward, through L1 and past it, by average list: 3M tets of a scene, 300 x 300, 2742: 1049 us, 846; 6.7M, 600 x 600,
+// 1634: 736, 627; 21M, 1080p, 1886: 2166, 2024; 6.7M, 1080p, 1083: 1518, 1501; 1.2M in clusters, 300 x 300, 909: 304, 291).  Short
+// lists live of it (0.6M, 800 x 800, 230: 375, 414; 1.2M, 600 x 600, 415: 400, 459); between 650 and 880 it is the same.
+// The line lies there for larger tiles too, where 4 or 16 units walk one list: 8 x 8, 1M tets, 640 x 640, 922: 388, 359; 320 x 320,
+// 1524: 437, 412; 6.7M, 1080p, 1380: 1712, 1644; 0.6M, 800 x 800, 343: 404, 539; 16 x 16, 1.3M, 800 x 800, 1300: 949, 936; 6.7M, 1080p,
+// 2203: 2419, 2321; 0.3M and 0.6M, 800 x 800, 544 and 660: 522 and 504, 613 and 641.
 static bool lines_past_l1(int64_t tiles, int64_t n_list) { return n_list >= 800 * tiles; }
 
 int rm_launch_forward(const int32_t* list, const int32_t* ranges, const float* records, const RmCamera* cam,

@@ -124,24 +124,18 @@ struct PendingInfo {
   Tensor block;
   at::cuda::CUDAEvent written;
   c10::cuda::CUDAStream stream;
-  bool recorded = false, arrived = false;
+  bool arrived = false;
 
   explicit PendingInfo(c10::cuda::CUDAStream s)
       : block(at::empty({3}, at::TensorOptions().dtype(at::kLong).pinned_memory(true))), stream(s) {}
   ~PendingInfo() {
     if (!arrived) cudaStreamSynchronize(stream.stream());
   }
-  void record() {
-    written.record(stream);
-    recorded = true;
-  }
+  void record() { written.record(stream); }
   // The one host synchronisation of a frame: (list entries, region pairs, visible tets, status bits).  What was enqueued behind
   // the info block is not waited for.
   std::tuple<int64_t, int64_t, int64_t, int64_t> wait() {
-    if (!arrived) {
-      if (recorded) written.synchronize();
-      else stream.synchronize();
-    }
+    if (!arrived) written.synchronize();
     arrived = true;
     const RmBinInfo* r = ptr<RmBinInfo>(block);
     return {r->n_keys, r->n_region_keys, r->n_visible, r->status};
