@@ -29,32 +29,48 @@ def _frame(s, ahead, grad=True):
     return pkg, v.grad, c.grad
 
 
+@pytest.fixture
+def packed_ahead(monkeypatch):
+    """Of every call of pack_ahead that `render` makes, whether it has packed."""
+    from radiance_meshes_b200 import render as module
+    calls, pack_ahead = [], module.pack_ahead
+
+    def spy(*args):
+        packed = pack_ahead(*args)
+        calls.append(packed is not None)
+        return packed
+    monkeypatch.setattr(module, "pack_ahead", spy)
+    return calls
+
+
 @pytest.mark.parametrize("change", [{}, {"cell": lambda t: t.double()}, {"cell": lambda t: t.t().contiguous().t()},
                                     {"indices": lambda t: t.long()}, {"vertices": lambda t: t.double()},
                                     {"indices": lambda t: t[:1]}, {"tcam": lambda c: dict(c, tile_rows=None)}])
 @pytest.mark.parametrize("grad", [True, False])
-def test_same_frame(cuda_lib, change, grad):
+def test_same_frame(cuda_lib, packed_ahead, change, grad):
     """Types, orders and sizes that the blend takes: the same bits, and gradients that differ by the order of their sums (the
     atomics of some hundred tets a vertex: 1e-5)."""
-    if "indices" in change:
-        change = dict(change, cell=change.get("cell", lambda t: t))
     s = _inputs(**change)
     s["cell"] = s["cell"][:s["indices"].shape[0]]
-    (a, va, ca), (b, vb, cb) = _frame(s, True, grad), _frame(s, False, grad)
+    a, va, ca = _frame(s, True, grad)
+    assert packed_ahead == [True]
+    b, vb, cb = _frame(s, False, grad)
+    assert packed_ahead == [True]
     for k in ("image", "distortion_img", "sorted_tetra_idx", "tile_ranges", "mask"):
         assert torch.equal(a[k], b[k]), k
     if grad:
         assert float((va - vb).norm()) <= 1e-5 * float(vb.norm()) and float((ca - cb).norm()) <= 1e-5 * float(cb.norm())
 
 
-@pytest.mark.parametrize("change,error", [({"cell": lambda t: t[:, :4].contiguous()}, AssertionError),
-                                          ({"vertices": lambda t: t * float("nan")}, AssertionError),
-                                          ({"indices": lambda t: t + 10_000}, IndexError)])
-def test_what_was_refused_stays_refused(cuda_lib, change, error):
+@pytest.mark.parametrize("change,error,packs", [({"cell": lambda t: t[:, :4].contiguous()}, AssertionError, False),
+                                                ({"vertices": lambda t: t * float("nan")}, AssertionError, True),
+                                                ({"indices": lambda t: t + 10_000}, IndexError, True)])
+def test_what_was_refused_stays_refused(cuda_lib, packed_ahead, change, error, packs):
     s = _inputs(**change)
     for ahead in (True, False):
         with pytest.raises(error):
             _frame(s, ahead, grad=False)
+    assert packed_ahead == [packs]
     torch.cuda.synchronize()
     good, _, _ = _frame(_inputs(), True, grad=False)  # a frame given up leaves nothing behind
     assert np.isfinite(good["image"].cpu().numpy()).all()
@@ -84,11 +100,12 @@ def _peak(call):
 
 
 @pytest.mark.parametrize("grad", [False, True])
-def test_large_mesh_needs_no_more_memory(cuda_lib, grad):
-    """One tet above the limit: records beside the list scratch would be 144 MB more at the peak of a frame alone."""
+def test_large_mesh_needs_no_more_memory(cuda_lib, packed_ahead, grad):
+    """One tet above the limit: records beside the list scratch would be 46 MB more at the peak of a frame alone."""
     from radiance_meshes_b200 import raster
     s = _many_tets(raster.PACK_AHEAD_TETS + 1)
     _frame(s, True, grad)
+    assert packed_ahead == [True] * grad
     assert _peak(lambda: _frame(s, True, grad)) <= _peak(lambda: _frame(s, False, grad)) + 2**20
 
 
